@@ -11,12 +11,14 @@
 #include <cstring>
 #include <mutex>
 #include <string>
+#include <tuple>
 #include <vector>
 
 #include "../../include/meanas_fdfd.h"
 #include "fdfd_csr.cuh"
 #include "fdfd_fdtd.cuh"
 #include "fdfd_ops.cuh"
+#include "fdfd_resident.cuh"
 
 using namespace fdfd;
 
@@ -105,6 +107,14 @@ struct Tiling {
   long long nblocks;
 };
 
+// Resident solve of one precision: brick split, cells per thread, launch shape (grid 0: the
+// grid does not fit).
+struct ResidentPlan {
+  Bricks bk;
+  int k, grid;
+  size_t smem;
+};
+
 struct GraphEntry {
   int kind;
   const void* a;
@@ -134,6 +144,8 @@ struct fdfd_plan {
   KState* h_state;         // pinned
   std::vector<GraphEntry> graphs;
   int launches;            // kernel launches counter for the current call
+  ResidentPlan res_cocg;   // complex128 COCG
+  size_t smem_optin;       // shared memory a CTA may ask for
   // optional per-kernel timing (fdfd_solve_opts.profile)
   bool profiling;
   std::vector<cudaEvent_t> ev_pool;
@@ -317,6 +329,70 @@ static int launch_point(fdfd_plan* P, const Geo<R>& g0, int precision, const Op&
   return 0;
 }
 
+// ------------------------------------------------------------------ resident solves
+static constexpr int RES_NT = 512;     // 128 registers a thread (576 to 768 threads spill more and are slower)
+static constexpr int RES_CHUNK = 256;  // iterations per launch: a millisecond or two between polls
+
+// The brick split with the least work on the largest brick among those of at most one CTA
+// per SM that fit the shared memory with `nshell` shell vectors, one or two own cells per
+// thread.  Work: an own cell takes part in every pass, a shell cell and an H cell in one or
+// two.
+template <typename R>
+static ResidentPlan plan_resident(const fdfd_plan* P, int nshell, size_t smem_max) {
+  ResidentPlan best{};
+  long long best_cost = -1;
+  const int most = std::min(P->nsm, RES_CTAS);
+  for (int nx = 1; nx <= std::min(P->X, most); ++nx) {
+    for (int ny = 1; ny <= std::min(P->Y, most / nx); ++ny) {
+      for (int nz = 1; nz <= (P->flat ? 1 : std::min(P->Z, most / (nx * ny))); ++nz) {
+        const int bx = (P->X + nx - 1) / nx, by = (P->Y + ny - 1) / ny, bz = (P->Z + nz - 1) / nz;
+        const long long own = (long long)bx * by * bz;
+        int k = 1;
+        if (own > RES_NT) k = 2;
+        if ((long long)((bx + k - 1) / k) * by * bz > RES_NT) continue;
+        const int kz = P->flat ? 0 : 1;
+        const long long box = (long long)(bx + 2) * (by + 2) * (bz + 2 * kz);
+        const long long hbox = (long long)(bx + 1) * (by + 1) * (bz + kz);
+        const size_t smem = resident_layout<R>(nshell, P->flat, bx, by, bz).total;
+        if (smem > smem_max) continue;
+        const long long cost = own + box + hbox;
+        if (best_cost < 0 || cost < best_cost) {
+          best_cost = cost;
+          best = ResidentPlan{Bricks{nx, ny, nz, bx, by, bz}, k, nx * ny * nz, smem};
+        }
+      }
+    }
+  }
+  return best;
+}
+
+template <class... KArgs, class... Args>
+static int launch_resident(fdfd_plan* P, void (*kern)(KArgs...), const ResidentPlan& rp, cudaStream_t s,
+                           Args... args) {
+  // (the attribute is set once per kernel: to the most any plan may ask for)
+  if (int rc = ensure_smem(kern, P->smem_optin)) return rc;
+  std::tuple<KArgs...> a(args...);
+  std::apply(
+      [&](auto&... v) {
+        void* ptr[] = {(void*)&v...};
+        cudaLaunchCooperativeKernel((const void*)kern, dim3(rp.grid), dim3(RES_NT), ptr, rp.smem, s);
+      },
+      a);
+  P->launches++;
+  CKL();
+  return 0;
+}
+
+template <bool FLAT>
+static int launch_cocg_resident(fdfd_plan* P, cx<double>* r, cx<double>* p, cx<double>* x, Word* surface, KState* st,
+                                ResidentScratch* gs, unsigned long long tag, int nit, cudaStream_t s) {
+  const ResidentPlan& rp = P->res_cocg;
+  CK(cudaMemsetAsync(gs->counter, 0, sizeof(gs->counter), s));
+  if (rp.k == 1)
+    return launch_resident(P, k_cocg_resident<RES_NT, 1, FLAT>, rp, s, P->g64, rp.bk, r, p, x, surface, st, gs, tag, nit);
+  return launch_resident(P, k_cocg_resident<RES_NT, 2, FLAT>, rp, s, P->g64, rp.bk, r, p, x, surface, st, gs, tag, nit);
+}
+
 #define TRY(x)                 \
   do {                         \
     int rc_ = (x);             \
@@ -483,6 +559,13 @@ extern "C" int fdfd_plan_create(const fdfd_grid_desc* d, void* ws, size_t ws_byt
   cudaGetDevice(&dev);
   cudaDeviceGetAttribute(&P->nsm, cudaDevAttrMultiProcessorCount, dev);
   if (P->nsm <= 0) P->nsm = 148;
+  {
+    int coop = 0, optin = 0;
+    cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, dev);
+    cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev);
+    P->smem_optin = (size_t)optin;
+    if (coop) P->res_cocg = plan_resident<double>(P, 1, P->smem_optin);
+  }
   auto cleanup = [&](int rc) {
     delete P;
     return rc;
@@ -573,7 +656,7 @@ extern "C" int fdfd_apply(fdfd_plan* P, int32_t op, int32_t precision, const voi
 // the inner precision.  COCG also needs r, q, P0, P1, which its breakdown
 // fallback (complex128 BiCGSTAB) reuses as R0, R1, P0, P1.
 struct SolveLayout {
-  size_t state, ticket, partials, resid, b, e2, cocg[4], inner[8], total;
+  size_t state, ticket, scratch, partials, resid, b, e2, cocg[4], inner[8], total;
 };
 
 static void solve_layout(const fdfd_plan* P, const fdfd_solve_opts* o, SolveLayout* L) {
@@ -587,6 +670,8 @@ static void solve_layout(const fdfd_plan* P, const fdfd_solve_opts* o, SolveLayo
   off += 256;
   L->resid = off;
   off += 256;
+  L->scratch = off;
+  off += align256(sizeof(ResidentScratch));
   L->partials = off;
   off += align256((size_t)max_blocks(P) * 8 * sizeof(double));
   L->b = off;
@@ -744,6 +829,9 @@ struct SolveCtx {
   KState* st;      // outer state
   KState* st_in;   // inner state
   RedBuf rb;
+  ResidentScratch* scratch;  // of resident solves, and the number of their last exchange
+  unsigned long long tag;
+  Word* surface;   // their surface words (two buffers of all cells), null: no room for them
   cx<double>* b;
   cx<double>* x;   // the caller's E
   cx<double>* e2;  // partner of E for the refinement ping-pong
@@ -877,12 +965,25 @@ static int cocg_loop(SolveCtx& c, cx<double>* r, cx<double>* q, cx<double>* P0, 
     }
     return 0;
   };
+  // Every grid that fits runs resident: it is 2 to 4 times faster than the two launches up to
+  // the largest that do (52^3 and 380^2 cells, see k_cocg_resident).  The two-launch form
+  // stays for larger grids, for profiling (which times its passes) and where the caller's
+  // workspace has no room for the surface words (the fallback of the mixed solver).
+  const bool resident = c.surface && P->res_cocg.grid > 0 && !P->profiling;
   int restarts = 0;
   for (;;) {
     CK(cudaMemcpyAsync(P->h_state, st, sizeof(KState), cudaMemcpyDeviceToHost, s));
     CK(cudaStreamSynchronize(s));
     const int left = maxiter - c.iters;
-    if (P->h_state->status == ST_RUNNING && left > 0) {
+    if (resident && P->h_state->status == ST_RUNNING && left > 0) {
+      const int nit = o->chunk > 0 ? o->chunk : RES_CHUNK;
+      TRY(drive(P, st, nit, left, s, [&]() -> int {
+        const unsigned long long tag = c.tag;
+        c.tag += (unsigned long long)nit;
+        return P->flat ? launch_cocg_resident<true>(P, r, P0, x, c.surface, st, c.scratch, tag, nit, s)
+                       : launch_cocg_resident<false>(P, r, P0, x, c.surface, st, c.scratch, tag, nit, s);
+      }));
+    } else if (P->h_state->status == ST_RUNNING && left > 0) {
       TRY(drive(P, st, chunk, left, s, [&]() -> int {
         if (o->use_graph && !P->profiling) {
           P->launches += 2 * chunk;
@@ -891,12 +992,15 @@ static int cocg_loop(SolveCtx& c, cx<double>* r, cx<double>* q, cx<double>* P0, 
         return enqueue(s);
       }));
     }
-    OpCocgFinal<double> fin{P0, P1, x, N, st};
-    TRY(launch_point<double>(P, P->g64, 0, fin, rb, s));
+    if (!resident) {  // (a resident launch leaves no update owed)
+      OpCocgFinal<double> fin{P0, P1, x, N, st};
+      TRY(launch_point<double>(P, P->g64, 0, fin, rb, s));
+    }
     CK(cudaMemcpyAsync(P->h_state, st, sizeof(KState), cudaMemcpyDeviceToHost, s));
     CK(cudaStreamSynchronize(s));
     c.iters += P->h_state->iter;
     c.status = P->h_state->status;
+    if (c.status == ST_TIMEOUT) return set_err(FDFD_ERR_CUDA, "a CTA of a resident solve did not arrive in time");
     if (c.status == ST_RUNNING) c.status = ST_MAXITER;
     if (c.status != ST_BREAKDOWN || restarts >= 8 || c.iters >= maxiter) break;
     // Breakdown: the unconjugated form cancelled (for example a source whose
@@ -965,6 +1069,9 @@ extern "C" int fdfd_solve(fdfd_plan* P, const fdfd_solve_opts* o, const void* J,
   unsigned int* ticket = (unsigned int*)(base + L.ticket);
   double* d_res = (double*)(base + L.resid);
   c.rb = RedBuf{(double*)(base + L.partials), ticket};
+  c.scratch = (ResidentScratch*)(base + L.scratch);
+  c.tag = 0;
+  c.surface = nullptr;
   c.b = (cx<double>*)(base + L.b);
   c.x = (cx<double>*)E;
   c.e2 = (cx<double>*)(base + L.e2);
@@ -988,6 +1095,7 @@ extern "C" int fdfd_solve(fdfd_plan* P, const fdfd_solve_opts* o, const void* J,
   KState h = make_state(o, c.crit, maxiter, o->history);
   *P->h_state = h;
   CK(cudaMemsetAsync(ticket, 0, sizeof(unsigned int), s));
+  CK(cudaMemsetAsync(c.scratch, 0, sizeof(ResidentScratch), s));
   CK(cudaMemcpyAsync(c.st, P->h_state, sizeof(KState), cudaMemcpyHostToDevice, s));
   // right-hand side (and guess) in the solve space; E holds the iterate
   {
@@ -1010,6 +1118,11 @@ extern "C" int fdfd_solve(fdfd_plan* P, const fdfd_solve_opts* o, const void* J,
     cx<double>* q = (cx<double>*)(base + L.cocg[1]);
     cx<double>* P0 = (cx<double>*)(base + L.cocg[2]);
     cx<double>* P1 = (cx<double>*)(base + L.cocg[3]);
+    if (P->res_cocg.grid > 0) {
+      // V0, V1, T and D of the fallback lie one after another and are free until it runs
+      c.surface = (Word*)B.V0;
+      CK(cudaMemsetAsync(c.surface, 0, 4 * vbytes128, s));
+    }
     TRY(cocg_loop(c, r, q, P0, P1, B, o->has_guess != 0, 0));
   } else if (o->method == FDFD_METHOD_MIXED) {
     const double eta = o->inner_rtol > 0 ? o->inner_rtol : 1e-2;
