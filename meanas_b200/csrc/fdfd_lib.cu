@@ -145,6 +145,7 @@ struct fdfd_plan {
   std::vector<GraphEntry> graphs;
   int launches;            // kernel launches counter for the current call
   ResidentPlan res_cocg;   // complex128 COCG
+  ResidentPlan res_bs;     // complex64 BiCGSTAB
   size_t smem_optin;       // shared memory a CTA may ask for
   // optional per-kernel timing (fdfd_solve_opts.profile)
   bool profiling;
@@ -393,6 +394,19 @@ static int launch_cocg_resident(fdfd_plan* P, cx<double>* r, cx<double>* p, cx<d
   return launch_resident(P, k_cocg_resident<RES_NT, 2, FLAT>, rp, s, P->g64, rp.bk, r, p, x, surface, st, gs, tag, nit);
 }
 
+template <bool FLAT>
+static int launch_bicgstab_resident(fdfd_plan* P, cx<float>* r, cx<float>* p, cx<float>* x, Word* surface,
+                                    unsigned seed, KState* st, ResidentScratch* gs, unsigned long long tag, int nit,
+                                    cudaStream_t s) {
+  const ResidentPlan& rp = P->res_bs;
+  CK(cudaMemsetAsync(gs->counter, 0, sizeof(gs->counter), s));
+  if (rp.k == 1)
+    return launch_resident(P, k_bicgstab_resident<RES_NT, 1, FLAT>, rp, s, P->g32, rp.bk, r, p, x, surface, seed, st,
+                           gs, tag, nit);
+  return launch_resident(P, k_bicgstab_resident<RES_NT, 2, FLAT>, rp, s, P->g32, rp.bk, r, p, x, surface, seed, st, gs,
+                         tag, nit);
+}
+
 #define TRY(x)                 \
   do {                         \
     int rc_ = (x);             \
@@ -564,7 +578,10 @@ extern "C" int fdfd_plan_create(const fdfd_grid_desc* d, void* ws, size_t ws_byt
     cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, dev);
     cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev);
     P->smem_optin = (size_t)optin;
-    if (coop) P->res_cocg = plan_resident<double>(P, 1, P->smem_optin);
+    if (coop) {
+      P->res_cocg = plan_resident<double>(P, 1, P->smem_optin);
+      if (P->has32) P->res_bs = plan_resident<float>(P, 4, P->smem_optin);
+    }
   }
   auto cleanup = [&](int rc) {
     delete P;
@@ -910,19 +927,42 @@ static int refine_loop(SolveCtx& c, const Geo<RI>& gi, int prec, BsBufs B, doubl
       }
       return 0;
     };
+    bool resident = false;
+    if constexpr (sizeof(RI) == 4) {
+      // As for COCG, every grid that fits runs resident.  r, t and x keep their vectors (t's
+      // holds p between launches); the five between lie one after another and hold the
+      // surface words (96 of their 120 bytes per cell).
+      resident = P->res_bs.grid > 0 && !P->profiling;
+      if (resident) {
+        Word* surface = (Word*)B.R1;
+        if (local_outer == 1) CK(cudaMemsetAsync(surface, 0, 5 * vb, s));
+        const int nit = c.o->chunk > 0 ? c.o->chunk : RES_CHUNK;
+        TRY(drive(P, sti, nit, hi.maxiter, s, [&]() -> int {
+          const unsigned long long tag = c.tag;
+          c.tag += (unsigned long long)nit;
+          return P->flat ? launch_bicgstab_resident<true>(P, (cx<RI>*)B.R0, (cx<RI>*)B.T, D, surface, seed, sti,
+                                                          c.scratch, tag, nit, s)
+                         : launch_bicgstab_resident<false>(P, (cx<RI>*)B.R0, (cx<RI>*)B.T, D, surface, seed, sti,
+                                                           c.scratch, tag, nit, s);
+        }));
+      }
+    }
     // the shadow seed is baked into the batch, so graphs are keyed by it too
-    TRY(drive(P, sti, chunk, hi.maxiter, s, [&]() -> int {
+    if (!resident) TRY(drive(P, sti, chunk, hi.maxiter, s, [&]() -> int {
       if (c.o->use_graph && !P->profiling) {
         P->launches += 2 * chunk;
         return graph_batch(P, kind + 16 * (local_outer % 8), c.ws, c.x, chunk, s, enqueue);
       }
       return enqueue(s);
     }));
-    OpBsFinal<RI> fin{B, N, sti};
-    TRY(launch_point<RI>(P, gi, prec, fin, rb, s));
+    if (!resident) {
+      OpBsFinal<RI> fin{B, N, sti};
+      TRY(launch_point<RI>(P, gi, prec, fin, rb, s));
+    }
     CK(cudaMemcpyAsync(P->h_state, sti, sizeof(KState), cudaMemcpyDeviceToHost, s));
     CK(cudaStreamSynchronize(s));
     c.iters += P->h_state->iter;
+    if (P->h_state->status == ST_TIMEOUT) return set_err(FDFD_ERR_CUDA, "a CTA of a resident solve did not arrive in time");
     if (P->h_state->status == ST_NONFINITE) { c.status = ST_NONFINITE; break; }
     have_d = true;
   }

@@ -12,8 +12,8 @@
 // chain of plane loads per CTA and a last-CTA reduction tail in each of its two kernels,
 // all of it latency.
 //
-// Exchange (fdfd_resident.cuh measured the forms at 148 CTAs, cycles per exchange of one
-// sum, the block sum not counted): every CTA polling every CTA's word 6400; release /
+// Exchange (the forms measured at 148 CTAs, cycles per exchange of one or two sums, the
+// block sum not counted): every CTA polling every CTA's word 6400; release /
 // acquire around a counter and plain partial sums 5800 (the fences wait for all stores in
 // flight and empty the L1); a counter without fences and tagged words 2000, which is the
 // one taken.  A CTA stores a partial sum together with the number of the exchange in one
@@ -700,6 +700,262 @@ __global__ void __launch_bounds__(NT, 1)
     st->beta = {beta.re, beta.im};
     st->iter = iter;
     st->pending = 0;
+    st->status = status;
+  }
+}
+
+// ------------------------------------------------------------------ BiCGSTAB
+// `nit` iterations of the complex64 BiCGSTAB of fdfd_ops.cuh (OpBsP / OpBsS: the same
+// recurrences and tests) with r, p, v, t and x of a thread's K own cells in registers, r, p,
+// v and t of the shell and the operator's input U in shared memory:
+//   v = A0 p                own cells; surface cells also to their words   -> (rh, v)
+//   s = r - alpha v         own cells and shell (v of the shell from the words)
+//   t = A0 s                own cells, words                -> (t, s), |t|^2, (rh, t), |s|^2
+//   x += alpha p + omega s, r = s - omega t, p = r + beta (p - omega v)
+// A state with pending = 2 goes on from r and p in memory; otherwise p starts as r.  Both
+// shells are read before the sums that their writers wait for, so each product has one
+// buffer of 3 N words.
+//
+// Measured per iteration, two launches / resident: 16^3 29.6 / 7.6 us, 40^3 33.6 / 10.2,
+// 52^3 (the largest cube that fits) 44.2 / 15.1; flat 128^2 29.7 / 7.4, 380^2 39.6 / 10.7.
+// Bound as COCG is: two exchanges, then shared-memory bandwidth on full bricks.
+template <int NT, int K, bool FLAT>
+__global__ void __launch_bounds__(NT, 1)
+    k_bicgstab_resident(const Geo<float> g, const Bricks bk, cx<float>* r, cx<float>* p, cx<float>* x, Word* surface,
+                        unsigned seed, KState* st, ResidentScratch* gs, unsigned long long tag0, int nit) {
+  using R = float;
+  using C = cx<R>;
+  if (ld_status(st) != ST_RUNNING) return;
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  const ResidentLayout L = resident_layout<R>(4, FLAT, bk.bx, bk.by, bk.bz);
+  Brick<R, FLAT> B;
+  B.init(g, bk);
+  C* U = reinterpret_cast<C*>(smem_raw);
+  const int nshell = B.box - B.own;
+  C* Rs = reinterpret_cast<C*>(smem_raw + L.shell_vec);
+  C* Ps = Rs + 3 * nshell;
+  C* Vs = Ps + 3 * nshell;
+  C* Ts = Vs + 3 * nshell;
+  C* Hs = reinterpret_cast<C*>(smem_raw + L.h);
+  int2* shell = reinterpret_cast<int2*>(smem_raw + L.shell);
+  BrickTables<R> T;
+  T.carve(smem_raw + L.tables, bk.bx, bk.by, bk.bz);
+  double* red = reinterpret_cast<double*>(smem_raw + L.red);
+  double* sums = red + 32 * 8;
+  int* flags = reinterpret_cast<int*>(sums + 2 * RES_SUMS);
+  const int tid = threadIdx.x, N = g.N, YZ = g.Y * g.Z;
+  if (tid == 0) flags[0] = flags[1] = 0;
+  __syncthreads();
+  list_shell<R, NT, FLAT>(g, B, shell, &flags[0]);
+  T.load_all(g, B, NT);
+  const OwnCells<K> o = own_cells<K>(g, B);
+  __syncthreads();
+  const bool resume = st->pending == 2;
+  C rv[K][3], pv[K][3], vv[K][3], tv[K][3], xv[K][3], hv[K][3];
+#pragma unroll
+  for (int m = 0; m < K; ++m) {
+#pragma unroll
+    for (int c = 0; c < 3; ++c) {
+      rv[m][c] = pv[m][c] = vv[m][c] = tv[m][c] = xv[m][c] = hv[m][c] = czero<R>();
+      if (m >= o.n) continue;
+      const int idx = c * N + o.cell + m * YZ;
+      rv[m][c] = r[idx];
+      pv[m][c] = resume ? p[idx] : rv[m][c];
+      xv[m][c] = x[idx];
+      hv[m][c] = shadow<R>(idx, seed);
+    }
+  }
+  for (int e = tid; e < nshell; e += NT) {
+    const int cell = shell[e].y;
+#pragma unroll
+    for (int c = 0; c < 3; ++c) {
+      const C v = r[c * N + cell];
+      Rs[c * nshell + e] = v;
+      Ps[c * nshell + e] = resume ? p[c * N + cell] : v;
+    }
+  }
+  __syncthreads();  // other threads update these shell entries
+  const C w2 = *g.w2p;
+  const bool scribe = blockIdx.x == 0 && tid == 0;
+  const double tol2 = st->tol2;
+  const int maxiter = st->maxiter, stall_limit = st->stall_limit;
+  int iter = st->iter, status = ST_RUNNING, best_iter = st->best_iter;
+  double best_rr = st->best_rr, rr = st->rr;
+  dcx rho = st->rho;
+  const size_t nw = (size_t)N;
+  // shell entries go round from the first thread without own cells
+  const int items = ((B.lx + K - 1) / K) * B.ly * B.lz;
+  const int spare = tid >= items ? tid - items : tid - items + NT;
+  constexpr int NS = 2, NT6 = 6;
+  for (int it = 0; it < nit; ++it) {
+    const unsigned long long tag = tag0 + (unsigned long long)it + 1;
+    C alpha, omega, beta;
+#pragma unroll
+    for (int m = 0; m < K; ++m) {
+      if (m >= o.n) break;
+#pragma unroll
+      for (int c = 0; c < 3; ++c) U[c * B.box + o.pos + m * B.sy] = pv[m][c];
+    }
+    for (int e = spare; e < nshell; e += NT) {
+      const int pos = shell[e].x;
+#pragma unroll
+      for (int c = 0; c < 3; ++c) U[c * B.box + pos] = Ps[c * nshell + e];
+    }
+    __syncthreads();
+    brick_curl_e<R, NT, FLAT>(g, B, T, U, Hs);
+    __syncthreads();
+    brick_curl_h<R, K, FLAT>(g, B, T, U, Hs, w2, o, vv, surface, tag);
+    {
+      R a[2] = {R(0), R(0)};
+#pragma unroll
+      for (int m = 0; m < K; ++m) {
+#pragma unroll
+        for (int c = 0; c < 3; ++c) acc_cdot<R>(a, hv[m][c], vv[m][c]);
+      }
+      double acc[NS] = {(double)a[0], (double)a[1]};
+      sums_begin<NT, 0, NS>(acc, red, gs, tag);
+    }
+    // while the sums travel: v of the shell, in the warps that do not wait for a sum
+    for (int e = tid - 32 * NS; e >= 0 && e < nshell; e += NT - 32 * NS) {
+      C q[3];
+      if (!surface_load<R>(surface, nw, shell[e].y, q, tag)) flags[1] = 1;
+#pragma unroll
+      for (int c = 0; c < 3; ++c) Vs[c * nshell + e] = q[c];
+    }
+    if (!sums_end<0, NS>(sums, &flags[1], gs, tag, it + 1)) { status = ST_TIMEOUT; break; }
+    const dcx sigma = {sums[0], sums[1]};
+    if (!dfinite(sigma)) { status = ST_NONFINITE; break; }
+    if ((fmax(fabs(sigma.re), fabs(sigma.im)) <= 1e-300 && dabs(sigma) <= 1e-300) ||
+        (fmax(fabs(rho.re), fabs(rho.im)) <= 1e-300 && dabs(rho) <= 1e-300)) {
+      status = ST_BREAKDOWN;
+      break;
+    }
+    const dcx alpha_d = cdiv(rho, sigma);
+    alpha = from_d<R>(alpha_d);
+    const C malpha = mkc<R>(-alpha.re, -alpha.im);
+#pragma unroll
+    for (int m = 0; m < K; ++m) {
+      if (m >= o.n) break;
+#pragma unroll
+      for (int c = 0; c < 3; ++c) {
+        rv[m][c] = caxpy(malpha, vv[m][c], rv[m][c]);
+        U[c * B.box + o.pos + m * B.sy] = rv[m][c];
+      }
+    }
+    for (int e = spare; e < nshell; e += NT) {
+      const int pos = shell[e].x;
+#pragma unroll
+      for (int c = 0; c < 3; ++c) {
+        const C s = caxpy(malpha, Vs[c * nshell + e], Rs[c * nshell + e]);
+        Rs[c * nshell + e] = s;
+        U[c * B.box + pos] = s;
+      }
+    }
+    __syncthreads();
+    brick_curl_e<R, NT, FLAT>(g, B, T, U, Hs);
+    __syncthreads();
+    brick_curl_h<R, K, FLAT>(g, B, T, U, Hs, w2, o, tv, surface + SurfaceRows<R>::value * nw, tag);
+    {
+      R a[NT6] = {R(0), R(0), R(0), R(0), R(0), R(0)};
+#pragma unroll
+      for (int m = 0; m < K; ++m) {
+#pragma unroll
+        for (int c = 0; c < 3; ++c) {
+          acc_cdot<R>(a, tv[m][c], rv[m][c]);
+          a[2] += cabs2(tv[m][c]);
+          acc_cdot<R>(a + 3, hv[m][c], tv[m][c]);
+          a[5] += cabs2(rv[m][c]);
+        }
+      }
+      double acc[NT6];
+#pragma unroll
+      for (int q = 0; q < NT6; ++q) acc[q] = (double)a[q];
+      sums_begin<NT, NS, NT6>(acc, red, gs, tag);
+    }
+    for (int e = tid - 32 * NT6; e >= 0 && e < nshell; e += NT - 32 * NT6) {
+      C q[3];
+      if (!surface_load<R>(surface + SurfaceRows<R>::value * nw, nw, shell[e].y, q, tag)) flags[1] = 1;
+#pragma unroll
+      for (int c = 0; c < 3; ++c) Ts[c * nshell + e] = q[c];
+    }
+    if (!sums_end<NS, NT6>(sums + RES_SUMS, &flags[1], gs, tag, it + 1)) { status = ST_TIMEOUT; break; }
+    const double* q = sums + RES_SUMS;
+    const dcx ts = {q[0], q[1]}, rht = {q[3], q[4]};
+    const double tt = q[2], ss = q[5];
+    iter += 1;
+    if (!dfinite(ts) || !isfinite(tt) || !dfinite(rht) || !isfinite(ss)) {
+      status = ST_NONFINITE;
+      break;
+    }
+    const bool small_s = ss <= tol2 || tt <= 0.0;  // s small enough (or t vanished): finish with omega = 0
+    const double itt = small_s ? 0.0 : 1.0 / tt;
+    const dcx om = {ts.re * itt, ts.im * itt};
+    omega = from_d<R>(om);
+    rr = small_s ? ss : fmax(ss - (ts.re * ts.re + ts.im * ts.im) * itt, 0.0);
+    if (rr <= tol2) status = ST_CONVERGED;
+    else if (iter >= maxiter) status = ST_MAXITER;
+    if (status == ST_RUNNING && small_s) status = ST_BREAKDOWN;
+    if (status == ST_RUNNING) {
+      // stagnation: no 1 % improvement on the best residual for stall_limit iterations
+      if (rr < 0.98 * best_rr || iter == 1) {
+        best_rr = rr;
+        best_iter = iter;
+      } else if (stall_limit > 0 && iter - best_iter >= stall_limit) {
+        status = ST_BREAKDOWN;
+      }
+    }
+    beta = czero<R>();
+    if (status == ST_RUNNING) {
+      const dcx rho_new = {-(om.re * rht.re - om.im * rht.im), -(om.re * rht.im + om.im * rht.re)};
+      if ((fmax(fabs(om.re), fabs(om.im)) <= 1e-300 && dabs(om) <= 1e-300) ||
+          (fmax(fabs(rho_new.re), fabs(rho_new.im)) <= 1e-300 && dabs(rho_new) <= 1e-300)) {
+        status = ST_BREAKDOWN;
+      } else {
+        // beta = (rho_new / rho) (alpha / omega)
+        beta = from_d<R>(dmul(cdiv(rho_new, rho), cdiv(alpha_d, om)));
+        rho = rho_new;
+      }
+    }
+    const C momega = mkc<R>(-omega.re, -omega.im);
+#pragma unroll
+    for (int m = 0; m < K; ++m) {
+      if (m >= o.n) break;
+#pragma unroll
+      for (int c = 0; c < 3; ++c) {
+        xv[m][c] = caxpy(omega, rv[m][c], caxpy(alpha, pv[m][c], xv[m][c]));
+        rv[m][c] = caxpy(momega, tv[m][c], rv[m][c]);
+        pv[m][c] = caxpy(beta, caxpy(momega, vv[m][c], pv[m][c]), rv[m][c]);
+      }
+    }
+    if (status != ST_RUNNING) break;
+    for (int e = spare; e < nshell; e += NT) {
+#pragma unroll
+      for (int c = 0; c < 3; ++c) {
+        const int at = c * nshell + e;
+        const C rn = caxpy(momega, Ts[at], Rs[at]);
+        Rs[at] = rn;
+        Ps[at] = caxpy(beta, caxpy(momega, Vs[at], Ps[at]), rn);
+      }
+    }
+  }
+#pragma unroll
+  for (int m = 0; m < K; ++m) {
+    if (m >= o.n) break;
+#pragma unroll
+    for (int c = 0; c < 3; ++c) {
+      const int idx = c * N + o.cell + m * YZ;
+      x[idx] = xv[m][c];
+      p[idx] = pv[m][c];
+      r[idx] = rv[m][c];
+    }
+  }
+  if (scribe) {
+    st->rho = rho;
+    st->rr = rr;
+    st->best_rr = best_rr;
+    st->best_iter = best_iter;
+    st->iter = iter;
+    st->pending = 2;
     st->status = status;
   }
 }

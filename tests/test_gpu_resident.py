@@ -49,3 +49,89 @@ def test_cocg_iterates_match_the_two_launch_form(cuda, shape, masks, adjoint):
     assert numpy.allclose(info.history, ref.history, rtol=1e-6, atol=1e-12)
     E2, _ = op.solve(J, **kw)  # fixed order of all sums: the same bits again
     assert numpy.array_equal(E2.cpu().numpy(), E)
+
+
+MIXED = [(1, 1, 1), (2, 1, 3), (5, 4, 1), (3, 60, 7), (31, 33, 29), (48, 48, 48), (52, 52, 52), (57, 56, 57),
+         (128, 128, 1), (389, 380, 1), (410, 410, 1)]
+
+
+def _shadow(n, seed):
+    """The solver's hashed shadow vector (``shadow`` in fdfd_ops.cuh)."""
+    def mix(x):
+        for shift, mul in ((16, 0x7feb352d), (15, 0x846ca68b), (16, 1)):
+            x = (x ^ (x >> numpy.uint32(shift))) * numpy.uint32(mul)
+        return x
+    with numpy.errstate(over='ignore'):
+        a = mix(numpy.arange(n, dtype=numpy.uint32) ^ numpy.uint32(seed))
+        b = mix(a ^ numpy.uint32(((seed << 16) | (seed >> 16)) & 0xffffffff) ^ numpy.uint32(0x9e3779b9))
+    return (a * 2.0 ** -32 - 0.5) + 1j * (b * 2.0 ** -32 - 0.5)
+
+
+def _bicgstab(A, b, shadow, steps, dtype):
+    """The iterate after ``steps`` of BiCGSTAB from zero, vectors in ``dtype``, sums in FP64."""
+    def dot(u, v):
+        return complex(numpy.vdot(u.astype(complex), v.astype(complex)))
+    A, r, rh = A.astype(dtype), b.astype(dtype), shadow.astype(dtype)
+    x, p, rho = numpy.zeros_like(r), r.copy(), dot(rh, r)
+    for _ in range(steps):
+        v = A @ p
+        alpha = rho / dot(rh, v)
+        s = r - dtype(alpha) * v
+        t = A @ s
+        omega = dot(t, s) / dot(t, t).real
+        x = x + dtype(alpha) * p + dtype(omega) * s
+        r = s - dtype(omega) * t
+        rho_new = -omega * dot(rh, t)
+        beta = rho_new / rho * alpha / omega
+        rho = rho_new
+        p = r + dtype(beta) * (p - dtype(omega) * v)
+    return x.astype(complex)
+
+
+@pytest.mark.parametrize('masks', [False, True])
+@pytest.mark.parametrize('shape', MIXED, ids=str)
+def test_bicgstab_iterates_match_the_oracle(cuda, shape, masks):
+    """One and three iterations (the second launch goes on from the first one's state)
+    against the same recurrence in complex128 on the host.  How far complex64 takes an
+    iterate off depends on the problem, so the host's complex64 iterate sets the scale: ten
+    times its error and 1e-6 (sixteen roundings of 6e-8)."""
+    from meanas_b200.operators import GridOperator
+    from oracle import fdfd_oracle as O
+    p, J, _ = _problem(shape, masks, seed=1)
+    if numpy.prod(shape) < 8:
+        pytest.skip('three steps exhaust the Krylov space')
+    op = GridOperator(**p, device=cuda)
+    A = O.e_full_csr(p['omega'], p['dxes'], p['epsilon'], p['mu'], p['pec'], p['pmc'])
+    b = -1j * p['omega'] * J
+    if masks:
+        b = numpy.where(p['pec'] > 0, 0, b)
+    bn = numpy.linalg.norm(b)
+    for steps in (1, 3):
+        E, info = op.solve(J, method='mixed', rtol=1e-13, criterion='true', maxiter=steps, max_outer=1,
+                           inner_rtol=1e-6, chunk=2)
+        E = E.cpu().numpy()
+        # the seed of the first refinement step's shadow vector
+        ref, single = (bn * _bicgstab(A, b / bn, _shadow(len(b), 0x5eed5eed), steps, t)
+                       for t in (numpy.complex128, numpy.complex64))
+        assert info.iterations == steps
+        size = numpy.linalg.norm(ref)
+        scale = numpy.linalg.norm(single - ref) / size
+        assert numpy.linalg.norm(E - ref) <= (1e-6 + 10 * scale) * size, (steps, scale)
+        E2, _ = op.solve(J, method='mixed', rtol=1e-13, criterion='true', maxiter=steps, max_outer=1,
+                         inner_rtol=1e-6, chunk=2)
+        assert numpy.array_equal(E2.cpu().numpy(), E)  # fixed order of all sums
+
+
+@pytest.mark.parametrize('shape', [(24, 31, 19), (100, 90, 1), (40, 40, 40)], ids=str)
+def test_mixed_solution_matches_cocg(cuda, shape):
+    """Converged to 1e-11, several launches and refinements: the two methods' fields agree."""
+    from meanas_b200.operators import GridOperator
+    p, J, _ = _problem(shape, False, seed=2)
+    p['omega'] = p['omega'] * (1 - 0.25j)
+    p['epsilon'][:] = 2.0
+    op = GridOperator(**p, device=cuda)
+    E, info = op.solve(J, method='mixed', rtol=1e-11, criterion='true', chunk=40)
+    Er, ref = op.solve(J, method='cocg', rtol=1e-11, criterion='true')
+    assert info.converged and ref.converged and info.residual <= 1e-11 * 1.01
+    # both residuals are at 1e-11; the lossy operator's condition number is below 1e4
+    assert float((E - Er).norm()) <= 1e-7 * float(Er.norm())
