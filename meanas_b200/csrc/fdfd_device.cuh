@@ -352,7 +352,9 @@ struct StencilShape {
   static constexpr size_t off_h = off_u + sizeof(cx<R>) * (size_t)2 * 3 * BOX;
   static constexpr size_t off_xt = off_h + sizeof(cx<R>) * (size_t)3 * HH * HW;
   static constexpr int XT_STRIDE = 6;  // per plane: idxe, idxh, dxe, dxh, (|dxe|, |dxh|)
-  static constexpr size_t off_red = off_xt + sizeof(cx<R>) * (size_t)XT_STRIDE * (XC_MAX + 1);
+  // halo difference factors: 1/dy_e of rows j0-1, j0, ... and 1/dz_e of column k0-1 (TY + 2)
+  static constexpr size_t off_ht = off_xt + sizeof(cx<R>) * (size_t)XT_STRIDE * (XC_MAX + 1);
+  static constexpr size_t off_red = (off_ht + sizeof(cx<R>) * (size_t)(TY + 2) + 15) & ~(size_t)15;
   // per-thread sums of a finished plane block ([NRED][NT], in the accumulator type)
   static constexpr size_t off_blk = off_red + 64 * sizeof(double);
   // complex128 passes only (see PartitionedSums); complex64 passes keep one partial per CTA
@@ -365,7 +367,13 @@ struct StencilShape {
 // One work unit of a stencil pass: the x chunk `unit / (ntz * nty)` of the y/z tile
 // `unit % (ntz * nty)`.  Writes the unit's reduction partials (one per plane block); the
 // grid-wide sum and the op's finish() are the caller's.
-template <typename R, int TZ, int TY, bool FLAT, class Op>
+// MAT: the grid has mu or conductors.  Without them none of their code is in the plane step:
+// the passes are bound by instruction issue more than by their copies (which have landed
+// when a step waits for them), and code that is skipped still costs fetches and registers.
+// At 160x160x128, with and without the skipped code: COCG stencil pass 239 -> 208 us, P pass
+// 254 -> 241, S pass 111 -> 103, product 137 -> 101 (with the symmetriser's square roots out
+// of it, OpApply), complex64 product 88 -> 59.
+template <typename R, int TZ, int TY, bool FLAT, bool MAT, class Op>
 __device__ __forceinline__ void stencil_unit(const Geo<R>& g, const Op& o, RedBuf rb, int unit,
                                              unsigned char* smem_raw) {
   using S = StencilShape<R, TZ, TY, FLAT, Op::NB, Op::NO>;
@@ -376,6 +384,7 @@ __device__ __forceinline__ void stencil_unit(const Geo<R>& g, const Op& o, RedBu
   cx<R>* U = reinterpret_cast<cx<R>*>(smem_raw + S::off_u);         // [2][3][BOX]
   cx<R>* Hs = reinterpret_cast<cx<R>*>(smem_raw + S::off_h);        // [3][HH*HW]
   cx<R>* Xt = reinterpret_cast<cx<R>*>(smem_raw + S::off_xt);       // [XC+1][6]
+  cx<R>* Ht = reinterpret_cast<cx<R>*>(smem_raw + S::off_ht);       // [TY+2]
   using A = typename AccT<R>::type;
   A* shblk = reinterpret_cast<A*>(smem_raw + S::off_blk);         // [NRED][NT]
 
@@ -431,8 +440,8 @@ __device__ __forceinline__ void stencil_unit(const Geo<R>& g, const Op& o, RedBu
   const bool row_halo = (ty == 0);
   const bool col_halo = !FLAT && (ty == TY - 1) && (tz < TY);
   const int jr = wrapi(j0 + (col_halo ? tz : 0), g.Y);
-  const cx<R> idy_halo = row_halo ? g.idxe[1][jm] : (col_halo ? g.idxe[1][jr] : czero<R>());
-  const cx<R> idze_km = FLAT ? czero<R>() : g.idxe[2][km];
+  if (tid < TY + 2) Ht[tid] = tid <= TY ? g.idxe[1][wrapi(j0 - 1 + tid, g.Y)] : (FLAT ? czero<R>() : g.idxe[2][km]);
+  const int halo_off = row_halo ? jm * g.Z + kh : jr * g.Z + km;  // the halo H cell of this thread
 
   // per-plane x factors of this CTA's planes (plane x0-1 first) into shared memory
   for (int t = tid; t <= x1 - x0; t += NT) {
@@ -493,14 +502,14 @@ __device__ __forceinline__ void stencil_unit(const Geo<R>& g, const Op& o, RedBu
   };
   // convert the landed raw inputs of plane iw into U[buf]; own cells of the CTA's own
   // planes (own_plane) also run the op's convert_own
-  auto convert = [&](int buf, int iw, bool own_plane, A* acc_to) {
+  auto convert = [&](int buf, int iw, bool own_plane, A* acc_to, uint8_t mask0, uint8_t mask1) {
     const int base = (int)iw * YZ;
 #pragma unroll
     for (int sl = 0; sl < 2; ++sl) {
       const int pos = sl == 0 ? pos0 : pos1;
       if (pos < 0) continue;
       const int cell = base + (sl == 0 ? off0 : off1);
-      const uint8_t m = g.mask ? g.mask[cell] : (uint8_t)0;
+      const uint8_t m = MAT ? (sl == 0 ? mask0 : mask1) : (uint8_t)0;
 #pragma unroll
       for (int c = 0; c < 3; ++c) {
         cx<R> v[NB > 0 ? NB : 1];
@@ -520,19 +529,37 @@ __device__ __forceinline__ void stencil_unit(const Geo<R>& g, const Op& o, RedBu
     }
   };
 
-  // H-grid scaling pm * mu^-1 at a cell, per component
-  auto hscale = [&](int cell, cx<R>& hx, cx<R>& hy, cx<R>& hz) {
+  // PEC/PMC bits of the two slots' cells on plane iw
+  auto slot_masks = [&](int iw, uint8_t& m0, uint8_t& m1) {
+    m0 = m1 = 0;
+    if (MAT && g.mask) {
+      m0 = g.mask[iw * YZ + off0];
+      if (pos1 >= 0) m1 = g.mask[iw * YZ + off1];
+    }
+  };
+  // H-grid scaling pm * mu^-1 at a cell, per component: loaded ahead of its use
+  struct HScale {
+    R mi[3];
+    uint8_t m;
+  };
+  auto hscale_load = [&](int cell, HScale& h) {
+    if (!MAT) return;
     if (g.muinv) {
-      hx = g.muinv[cell] * hx;
-      hy = g.muinv[N + cell] * hy;
-      hz = g.muinv[2 * N + cell] * hz;
+#pragma unroll
+      for (int c = 0; c < 3; ++c) h.mi[c] = g.muinv[c * N + cell];
     }
-    if (g.mask) {
-      const uint8_t m = g.mask[cell];
-      if (m & 8u) hx = czero<R>();
-      if (m & 16u) hy = czero<R>();
-      if (m & 32u) hz = czero<R>();
+    h.m = g.mask ? g.mask[cell] : (uint8_t)0;
+  };
+  auto hscale = [&](const HScale& h, cx<R>& hx, cx<R>& hy, cx<R>& hz) {
+    if (!MAT) return;
+    if (g.muinv) {
+      hx = h.mi[0] * hx;
+      hy = h.mi[1] * hy;
+      hz = h.mi[2] * hz;
     }
+    if (h.m & 8u) hx = czero<R>();
+    if (h.m & 16u) hy = czero<R>();
+    if (h.m & 32u) hz = czero<R>();
   };
 
   // H = ce(u) on plane i at box position (bj, bk); cur/nxt = buffers of planes i, i+1
@@ -565,18 +592,23 @@ __device__ __forceinline__ void stencil_unit(const Geo<R>& g, const Op& o, RedBu
   // (own slots only until the barrier: the barrier publishes Xt, U[0] and U[1])
   issue(ip);
   cp_async_wait_all();
-  convert(0, ip, false, acc);
+  uint8_t m0, m1;
+  slot_masks(ip, m0, m1);
+  convert(0, ip, false, acc, m0, m1);
   issue(x0);
+  slot_masks(x0, m0, m1);
   cp_async_wait_all();
-  convert(1, x0, true, acc);
+  convert(1, x0, true, acc, m0, m1);
   __syncthreads();
   // plane x0+1 starts landing while the prologue H is computed
   issue(x0 + 1 == g.X ? 0 : x0 + 1);
   cx<R> hy_prev, hz_prev;
   {
     cx<R> hx, hy, hz;
+    HScale hs;
+    hscale_load((int)ip * YZ + (int)jc * g.Z + kc, hs);
     curl_e(0, 1, ty + 1, tz + KZ, idye, idze, Xt[0], hx, hy, hz);
-    hscale((int)ip * YZ + (int)jc * g.Z + kc, hx, hy, hz);
+    hscale(hs, hx, hy, hz);
     hy_prev = hy;
     hz_prev = hz;
   }
@@ -598,6 +630,13 @@ __device__ __forceinline__ void stencil_unit(const Geo<R>& g, const Op& o, RedBu
 #pragma unroll
       for (int c = 0; c < 3; ++c) e3[c] = g.eps[c * N + cell];
     }
+    // mu and the conductors' bits of this step, all in flight together; loaded where they are
+    // used, each cost a memory round trip (121x97x109 with mu and masks: product 101 -> 74 us,
+    // complex64 63 -> 40, COCG stencil pass 168 -> 154, P pass 169 -> 155, S pass 88 -> 77)
+    HScale hs_own, hs_halo;
+    hscale_load(cell, hs_own);
+    if (row_halo || col_halo) hscale_load(ibase + halo_off, hs_halo);
+    slot_masks(in1, m0, m1);
     // Plane i+1's raw inputs landed.  No barrier is needed here: every thread copies and
     // converts only its own Sbox/Sown slots, U[nxt] (plane i-1) was last read before the
     // previous step's Hs barrier, and Hs is rewritten only after the barrier below.
@@ -605,15 +644,8 @@ __device__ __forceinline__ void stencil_unit(const Geo<R>& g, const Op& o, RedBu
     constexpr bool PART = PartitionedSums<R>::value && Op::NRED > 0;
     const int rbm = (1 << g.rb_shift) - 1;
     const bool block_end = ((i + 1) & rbm) == 0 || (i + 1 == x1);
-    if constexpr (PART) convert(nxt, in1, i + 1 < x1, accn);
-    else convert(nxt, in1, i + 1 < x1, acc);
-    // The slots are free as soon as this thread has converted them.  Passes that wait for
-    // their copies (complex128, several inputs) start plane i+2 here, before the barriers of
-    // this step: COCG stencil pass at 160x160x128 239 -> 205 us.  The others are bound by
-    // shared-memory and issue slots and run 1 % slower that way, so they start it after the
-    // barrier.
-    constexpr bool EARLY = sizeof(R) == 8 && Op::NB + Op::NO > 1;
-    if (EARLY && i + 1 < x1) issue(in1 + 1 == g.X ? 0 : in1 + 1);
+    if constexpr (PART) convert(nxt, in1, i + 1 < x1, accn, m0, m1);
+    else convert(nxt, in1, i + 1 < x1, acc, m0, m1);
     __syncthreads();       // U[nxt] = u(i+1) ready for the neighbours' differences
     if constexpr (PART) {
       // plane i-1 ended a block (chunks start on block boundaries): its per-thread sums
@@ -621,28 +653,28 @@ __device__ __forceinline__ void stencil_unit(const Geo<R>& g, const Op& o, RedBu
       if (i > x0 && (i & ((1 << g.rb_shift) - 1)) == 0 && tid < 32)
         sum_block_partials<NT, Op::NRED>(shblk, rb, part_of((i >> g.rb_shift) - 1));
     }
-    if (!EARLY && i + 1 < x1) issue(in1 + 1 == g.X ? 0 : in1 + 1);
+    if (i + 1 < x1) issue(in1 + 1 == g.X ? 0 : in1 + 1);
     const cx<R>* xe = Xt + (i - x0 + 1) * S::XT_STRIDE;
     const cx<R> idxe_i = xe[0], idxh_i = xe[1];
     cx<R> hx, hy, hz;
     curl_e(cur, nxt, ty + 1, tz + KZ, idye, idze, idxe_i, hx, hy, hz);
-    hscale(cell, hx, hy, hz);
+    hscale(hs_own, hx, hy, hz);
     const int hp = (ty + 1) * HW + tz + KZ;
     Hs[0 * HH * HW + hp] = hx;
     Hs[1 * HH * HW + hp] = hy;
     Hs[2 * HH * HW + hp] = hz;
     if (row_halo) {  // low y halo row (j0-1)
       cx<R> ax, ay, az;
-      curl_e(cur, nxt, 0, tz + KZ, idy_halo, idze, idxe_i, ax, ay, az);
-      hscale(ibase + (int)jm * g.Z + kh, ax, ay, az);
+      curl_e(cur, nxt, 0, tz + KZ, Ht[0], idze, idxe_i, ax, ay, az);
+      hscale(hs_halo, ax, ay, az);
       Hs[0 * HH * HW + tz + KZ] = ax;
       Hs[1 * HH * HW + tz + KZ] = ay;
       Hs[2 * HH * HW + tz + KZ] = az;
     }
     if (col_halo) {  // low z halo column (k0-1), row j0 + tz
       cx<R> ax, ay, az;
-      curl_e(cur, nxt, tz + 1, 0, idy_halo, idze_km, idxe_i, ax, ay, az);
-      hscale(ibase + (int)jr * g.Z + km, ax, ay, az);
+      curl_e(cur, nxt, tz + 1, 0, Ht[1 + tz], Ht[TY + 1], idxe_i, ax, ay, az);
+      hscale(hs_halo, ax, ay, az);
       Hs[0 * HH * HW + (tz + 1) * HW] = ax;
       Hs[1 * HH * HW + (tz + 1) * HW] = ay;
       Hs[2 * HH * HW + (tz + 1) * HW] = az;
@@ -668,7 +700,7 @@ __device__ __forceinline__ void stencil_unit(const Geo<R>& g, const Op& o, RedBu
     hy_prev = hy;
     hz_prev = hz;
     if (active) {
-      const uint8_t m = g.mask ? g.mask[cell] : (uint8_t)0;
+      const uint8_t m = MAT ? hs_own.m : (uint8_t)0;
 #pragma unroll
       for (int c = 0; c < 3; ++c) {
         cx<R> v = y[c] - (e3[c] * w2) * u[c];
@@ -714,14 +746,14 @@ __device__ __forceinline__ unsigned int stencil_nparts(const Geo<R>& g) {
   return (unsigned int)((g.X + (1 << g.rb_shift) - 1) >> g.rb_shift) * (unsigned int)(g.ntz * g.nty);
 }
 
-template <typename R, int TZ, int TY, bool FLAT, int MINB, class Op>
+template <typename R, int TZ, int TY, bool FLAT, bool MAT, int MINB, class Op>
 __global__ void __launch_bounds__(TZ * TY, MINB) k_stencil(const Geo<R> g, Op op, RedBuf rb) {
   using S = StencilShape<R, TZ, TY, FLAT, Op::NB, Op::NO>;
   extern __shared__ __align__(16) unsigned char smem_raw[];
   if (op.skip()) return;
   Op o = op;
   o.prepare();
-  stencil_unit<R, TZ, TY, FLAT, Op>(g, o, rb, blockIdx.x, smem_raw);
+  stencil_unit<R, TZ, TY, FLAT, MAT, Op>(g, o, rb, blockIdx.x, smem_raw);
   if constexpr (Op::NRED > 0) {
     double sums[Op::NRED];
     double* shred = reinterpret_cast<double*>(smem_raw + S::off_red);

@@ -195,14 +195,13 @@ static void prof_collect(fdfd_plan* P, double* ms, int* cnt) {
 static constexpr int FLAT_TY = 256;
 
 // Resident CTAs per SM the stencil kernels are compiled for (register cap 65536 /
-// (256 threads x value)): complex64 passes carry less state than complex128 ones.
-template <typename R>
+// (256 threads x value)): complex64 passes carry less state than complex128 ones, and those
+// with one or two inputs less than the others (product 65.7 -> 61.6 us at 160x160x128, with
+// mu and masks at 121x97x109 56.9 -> 43.9).  Complex128 products at three CTAs spill: 104.7 ->
+// 134.0 us.
+template <typename R, class Op>
 struct MinBlocks {
-  static constexpr int value = 2;
-};
-template <>
-struct MinBlocks<float> {
-  static constexpr int value = 3;
+  static constexpr int value = sizeof(R) == 8 ? 2 : (Op::NB <= 2 ? 4 : 3);
 };
 static constexpr int TZ3 = 32, TY3 = 8;
 
@@ -279,25 +278,27 @@ static int ensure_smem(K kern, size_t bytes) {
   return 0;
 }
 
+template <typename R, bool FLAT, bool MAT, class Op>
+static int launch_stencil_as(fdfd_plan* P, const Tiling& t, const Geo<R>& g, const Op& op, RedBuf rb, cudaStream_t s) {
+  constexpr int TZ = FLAT ? 1 : TZ3, TY = FLAT ? FLAT_TY : TY3;
+  using Sh = StencilShape<R, TZ, TY, FLAT, Op::NB, Op::NO>;
+  auto kern = k_stencil<R, TZ, TY, FLAT, MAT, MinBlocks<R, Op>::value, Op>;
+  if (int rc = ensure_smem(kern, Sh::smem_bytes(Op::NRED))) return rc;
+  kern<<<(unsigned)t.nblocks, dim3(TZ, TY), Sh::smem_bytes(Op::NRED), s>>>(g, op, rb);
+  P->launches++;
+  CKL();
+  return 0;
+}
+
 template <typename R, class Op>
 static int launch_stencil(fdfd_plan* P, const Geo<R>& g0, int precision, const Op& op, RedBuf rb,
                           cudaStream_t s) {
   const Tiling t = make_tiling(P, precision);
   const Geo<R> g = geo_with(g0, t);
-  if (P->flat) {
-    using Sh = StencilShape<R, 1, FLAT_TY, true, Op::NB, Op::NO>;
-    auto kern = k_stencil<R, 1, FLAT_TY, true, MinBlocks<R>::value, Op>;
-    if (int rc = ensure_smem(kern, Sh::smem_bytes(Op::NRED))) return rc;
-    kern<<<(unsigned)t.nblocks, dim3(1, FLAT_TY), Sh::smem_bytes(Op::NRED), s>>>(g, op, rb);
-  } else {
-    using Sh = StencilShape<R, TZ3, TY3, false, Op::NB, Op::NO>;
-    auto kern = k_stencil<R, TZ3, TY3, false, MinBlocks<R>::value, Op>;
-    if (int rc = ensure_smem(kern, Sh::smem_bytes(Op::NRED))) return rc;
-    kern<<<(unsigned)t.nblocks, dim3(TZ3, TY3), Sh::smem_bytes(Op::NRED), s>>>(g, op, rb);
-  }
-  P->launches++;
-  CKL();
-  return 0;
+  const bool mat = g.muinv || g.mask;
+  if (P->flat)
+    return mat ? launch_stencil_as<R, true, true>(P, t, g, op, rb, s) : launch_stencil_as<R, true, false>(P, t, g, op, rb, s);
+  return mat ? launch_stencil_as<R, false, true>(P, t, g, op, rb, s) : launch_stencil_as<R, false, false>(P, t, g, op, rb, s);
 }
 
 template <typename K>
@@ -656,13 +657,15 @@ extern "C" int fdfd_apply(fdfd_plan* P, int32_t op, int32_t precision, const voi
   P->launches = 0;
   RedBuf rb{nullptr, nullptr};
   if (precision == FDFD_C128) {
-    OpApply<double> o{(const cx<double>*)x, (cx<double>*)y, op, P->g64};
-    return launch_stencil<double>(P, P->g64, 0, o, rb, s);
+    if (op == FDFD_OP_A0)
+      return launch_stencil<double>(P, P->g64, 0, OpApply<double, false>{(const cx<double>*)x, (cx<double>*)y, op, P->g64}, rb, s);
+    return launch_stencil<double>(P, P->g64, 0, OpApply<double, true>{(const cx<double>*)x, (cx<double>*)y, op, P->g64}, rb, s);
   }
   if (precision == FDFD_C64) {
     if (!P->has32) return set_err(FDFD_ERR_ARG, "fdfd_apply: plan built without FDFD_GRID_FP32");
-    OpApply<float> o{(const cx<float>*)x, (cx<float>*)y, op, P->g32};
-    return launch_stencil<float>(P, P->g32, 1, o, rb, s);
+    if (op == FDFD_OP_A0)
+      return launch_stencil<float>(P, P->g32, 1, OpApply<float, false>{(const cx<float>*)x, (cx<float>*)y, op, P->g32}, rb, s);
+    return launch_stencil<float>(P, P->g32, 1, OpApply<float, true>{(const cx<float>*)x, (cx<float>*)y, op, P->g32}, rb, s);
   }
   return set_err(FDFD_ERR_ARG, "fdfd_apply: bad precision %d", precision);
 }

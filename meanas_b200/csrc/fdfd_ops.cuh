@@ -132,7 +132,9 @@ __device__ __forceinline__ dcx csqrt_principal(dcx z) {
   return {b / (2.0 * t), copysign(t, z.im)};
 }
 
-template <typename R>
+// SYM false is mode 0 alone: without the square roots its plane step is a quarter of the
+// code.
+template <typename R, bool SYM>
 struct OpApply {
   static constexpr int NB = 1, NO = 0, NRED = 0;
   static constexpr bool NEEDS_W = false;
@@ -161,8 +163,9 @@ struct OpApply {
   }
   __device__ cx<R> make_u(const cx<R>* v, int idx, int c) const {
     cx<R> u = v[0];
+    if (!SYM) return u;
     if (mode == 2) u = cconj(u);
-    if (mode >= 1) {
+    {
       const cx<R> pl = pl_at(c, idx);
       // Pr = 1 / Pl
       const R d = cabs2(pl);
@@ -178,8 +181,8 @@ struct OpApply {
     for (int c = 0; c < 3; ++c) {
       const int idx = c * g.N + cell;
       cx<R> v = yv[c];
-      if (mode >= 1) v = pl_at(c, idx) * v;
-      if (mode == 2) v = cconj(v);
+      if (SYM) v = pl_at(c, idx) * v;
+      if (SYM && mode == 2) v = cconj(v);
       y[idx] = v;
     }
   }
