@@ -75,6 +75,12 @@ def _real_type(t: torch.Tensor) -> int:
     raise TypeError(f'FDTD fields must be float32 or float64, got {t.dtype}')
 
 
+def _on_device(e, h) -> bool:
+    """True when both fields are CUDA tensors the kernels can use as they are."""
+    return isinstance(e, torch.Tensor) and isinstance(h, torch.Tensor) and e.is_cuda and h.is_cuda and \
+        e.is_contiguous() and h.is_contiguous()
+
+
 class _Fields:
     """Device views of the caller's fields; numpy arrays are copied back on exit."""
 
@@ -108,10 +114,9 @@ class _Grid:
         self.lib = _lib.load()
         self._mats: dict[int, torch.Tensor] = {}
 
-    def desc(self, form: int, dt: float, field_type: int, psi_type: int = _lib.REAL32) -> _lib.FdtdDesc:
+    def desc(self, form: int, dt: float, psi_type: int = _lib.REAL32) -> _lib.FdtdDesc:
         d = _lib.FdtdDesc()
         d.shape[:] = self.shape
-        d.field_type = field_type
         d.psi_type = psi_type
         d.form = form
         d.dt = float(dt)
@@ -119,6 +124,42 @@ class _Grid:
             d.dxe[a] = self.dx[0][a].data_ptr()
             d.dxh[a] = self.dx[1][a].data_ptr()
         return d
+
+    def stepper(self, entry: str, desc: _lib.FdtdDesc, written: int) -> Callable:
+        """``step(e, h, epsilon, mu)`` running the half step ``entry`` with the descriptor (its
+        field type set to the fields') and the two materials' device tensors (or None).
+        ``written``: which of e, h it changes.
+
+        A step on small grids is a few microseconds of kernel, so the host side is kept to a
+        copy of the ready-made descriptor (a copy per call: several threads may step at
+        once), the two pointers and the launch.
+        """
+        fn = getattr(self.lib, entry)
+        dev, index = self.device, self.device.index
+        template = bytes(desc)
+        if index is None:
+            index = torch.cuda.current_device()
+
+        def step(e, h, epsilon: torch.Tensor | None, mu: torch.Tensor | None) -> None:
+            fields = None
+            if not _on_device(e, h):
+                fields = _Fields(dev, e, h)  # host arrays, or the error for unusable tensors
+                e, h = fields.dev
+            d = _lib.FdtdDesc.from_buffer_copy(template)
+            d.field_type = _real_type(e)
+            if epsilon is not None:
+                d.epsilon = epsilon.data_ptr()
+            if mu is not None:
+                d.mu = mu.data_ptr()
+            if torch.cuda.current_device() == index:
+                rc = fn(C.byref(d), e.data_ptr(), h.data_ptr(), _stream_handle())
+            else:
+                with torch.cuda.device(dev):
+                    rc = fn(C.byref(d), e.data_ptr(), h.data_ptr(), _stream_handle())
+            _lib.check(rc)
+            if fields is not None:
+                fields.copy_back(written)
+        return step
 
     def material(self, m, name: str) -> torch.Tensor | None:
         """A float64 [3N] device copy of epsilon / mu (scalars broadcast), cached per object."""
@@ -146,16 +187,10 @@ def maxwell_h(dt: float, dxes, *, device: Any | None = None) -> Callable:
     """``f(e, h, mu=None)``: ``h -= dt * curl_forward(dxes[0])(e) [/ mu]`` in place; returns h
     (``meanas/fdtd/base.py:70-125``)."""
     grid = _Grid(dxes, device)
+    step = grid.stepper('fdfd_fdtd_update_h', grid.desc(_lib.FDTD_PLAIN, dt), 1)
 
     def mh_fun(e, h, mu=None):
-        f = _Fields(grid.device, e, h)
-        d = grid.desc(_lib.FDTD_PLAIN, dt, _real_type(f.dev[0]))
-        m = grid.material(mu, 'mu')
-        d.mu = m.data_ptr() if m is not None else None
-        with torch.cuda.device(grid.device):
-            _lib.check(grid.lib.fdfd_fdtd_update_h(C.byref(d), f.dev[0].data_ptr(), f.dev[1].data_ptr(),
-                                                   _stream_handle()))
-        f.copy_back(1)
+        step(e, h, None, grid.material(mu, 'mu'))
         return h
     return mh_fun
 
@@ -164,15 +199,10 @@ def maxwell_e(dt: float, dxes, *, device: Any | None = None) -> Callable:
     """``f(e, h, epsilon)``: ``e += dt * curl_back(dxes[1])(h) / epsilon`` in place; returns e
     (``meanas/fdtd/base.py:13-67``)."""
     grid = _Grid(dxes, device)
+    step = grid.stepper('fdfd_fdtd_update_e', grid.desc(_lib.FDTD_PLAIN, dt), 0)
 
     def me_fun(e, h, epsilon):
-        f = _Fields(grid.device, e, h)
-        d = grid.desc(_lib.FDTD_PLAIN, dt, _real_type(f.dev[0]))
-        d.epsilon = grid.material(epsilon, 'epsilon').data_ptr()
-        with torch.cuda.device(grid.device):
-            _lib.check(grid.lib.fdfd_fdtd_update_e(C.byref(d), f.dev[0].data_ptr(), f.dev[1].data_ptr(),
-                                                   _stream_handle()))
-        f.copy_back(0)
+        step(e, h, grid.material(epsilon, 'epsilon'), None)
         return e
     return me_fun
 
@@ -203,8 +233,8 @@ def updates_with_cpml(cpml_params: Sequence[Sequence[dict[str, Any] | None]], dt
             keep += [pe, ph, *psi]
             faces.append((a, pp, th, pe, ph, psi))
 
-    def desc(field_type: int) -> _lib.FdtdDesc:
-        d = grid.desc(_lib.FDTD_CPML, dt, field_type, psi_type)
+    def desc() -> _lib.FdtdDesc:
+        d = grid.desc(_lib.FDTD_CPML, dt, psi_type)
         for a, pp, th, pe, ph, psi in faces:
             f = d.face[a][pp]
             f.thickness = th
@@ -216,25 +246,17 @@ def updates_with_cpml(cpml_params: Sequence[Sequence[dict[str, Any] | None]], dt
 
     eps0 = grid.material(epsilon, 'epsilon')
 
+    d = desc()
+    step_e = grid.stepper('fdfd_fdtd_update_e', d, 0)
+    step_h = grid.stepper('fdfd_fdtd_update_h', d, 1)
+
     def update_E(e, h, epsilon=None) -> None:
-        f = _Fields(grid.device, e, h)
-        d = desc(_real_type(f.dev[0]))
-        d.epsilon = (grid.material(epsilon, 'epsilon') if epsilon is not None else eps0).data_ptr()
-        with torch.cuda.device(grid.device):
-            _lib.check(grid.lib.fdfd_fdtd_update_e(C.byref(d), f.dev[0].data_ptr(), f.dev[1].data_ptr(),
-                                                   _stream_handle()))
-        f.copy_back(0)
+        step_e(e, h, grid.material(epsilon, 'epsilon') if epsilon is not None else eps0, None)
 
     def update_H(e, h, mu=None) -> None:
-        f = _Fields(grid.device, e, h)
-        d = desc(_real_type(f.dev[0]))
-        m = None if mu is None or (not isinstance(mu, torch.Tensor) and numpy.all(numpy.asarray(mu) == 1)
-                                   and numpy.size(mu) <= 3) else grid.material(mu, 'mu')
-        d.mu = m.data_ptr() if m is not None else None
-        with torch.cuda.device(grid.device):
-            _lib.check(grid.lib.fdfd_fdtd_update_h(C.byref(d), f.dev[0].data_ptr(), f.dev[1].data_ptr(),
-                                                   _stream_handle()))
-        f.copy_back(1)
+        unit = mu is None or (not isinstance(mu, torch.Tensor) and numpy.all(numpy.asarray(mu) == 1)
+                              and numpy.size(mu) <= 3)
+        step_h(e, h, None, None if unit else grid.material(mu, 'mu'))
 
     update_E.psi = update_H.psi = keep  # keeps the device arrays alive with the closures
     return update_E, update_H

@@ -82,7 +82,9 @@ _TUNED: dict[tuple[int, tuple[int, int, int], str], int] = {}
 
 
 def _stream_handle() -> int:
-    return torch.cuda.current_stream().cuda_stream
+    # the handle alone: torch.cuda.current_stream() builds a stream object first (3.3 us, as
+    # long as a small kernel)
+    return torch._C._cuda_getCurrentRawStream(torch.cuda.current_device())
 
 
 class GridOperator:
