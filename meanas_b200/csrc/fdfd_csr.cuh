@@ -4,19 +4,27 @@
 // caller builds, e.g. from eh_full / h_full).  Complex128 CSR, 32-bit column indices,
 // 64-bit row pointers.
 //
-// SpMV: a group of LPR lanes per row walks the row's nonzeros and reduces with warp
-// shuffles; every warp handles 32 / LPR consecutive rows per step, so all lanes of a warp
-// run the same number of steps (the shuffles need whole warps).
+// SpMV: a group of LPR lanes per row walks the row's nonzeros, CSR_UNROLL steps at a time
+// with all their loads in flight together, and reduces with warp shuffles; every warp
+// handles 32 / LPR consecutive rows per step, so all lanes of a warp run the same number of
+// steps (the shuffles need whole warps).
 //
 // BiCGSTAB (complex, hashed shadow vector as in the stencil solver), three kernels per
-// iteration, the direction update and s = r - alpha v folded into the gathers of the two
-// products:
-//   CA: p = r + beta (p_old - omega v_old) on the own row, v = A p gathered with the same
-//       formula at the columns (ping-pong p / v buffers), sigma = (rh, v)      -> alpha
-//   CB: s = r - alpha v on the own row, t = A s gathered likewise, (t, s), |t|^2, |s|^2 -> omega
-//   CC: x += alpha p + omega s, r = s - omega t, (rh, r), |r|^2                  -> beta
-// Reductions are the deterministic grid reductions of the stencil engine; the scalars
-// (rho, alpha, omega, beta) stay in FP64 device state.
+// iteration; s = r - alpha v is formed where it is needed and never stored:
+//   CA: v = A p, sigma = (rh, v)                                        -> alpha
+//   CB: t = A (r - alpha v) with s formed at the columns, (t, s), |t|^2, |s|^2, (rh, s),
+//       (rh, t)                                                         -> omega, beta
+//   CC: x += alpha p + omega s, r = s - omega t, p = r + beta (p - omega v), |r|^2
+// Forming p and s in the gathers instead cost CA three gathers per nonzero.  Reductions are
+// the deterministic grid reductions of the stencil engine; the scalars (rho, alpha, omega,
+// beta) stay in FP64 device state.
+//
+// What bounds it: the latency of index load and gather, then L2 (a matrix of 20 bytes per
+// nonzero that stays there), and the reductions' tails.  Per iteration on the wave operator of
+// 40x36x32 cells (138 thousand rows, 12.9 nonzeros each): CA 33 -> 11.5 us, CB 26 -> 20, CC (one
+// lane in four worked) 20 -> 10.6, and 2 us between each two; launched so that a pass's CTAs
+// come up during the one before (pass_begin), 86 -> 43 us in all.  Four lanes per row: two are
+// as fast, eight 30 % slower; three CTAs per SM leave the registers for the unrolled loads.
 #pragma once
 #include "fdfd_ops.cuh"
 
@@ -46,12 +54,27 @@ __device__ __forceinline__ void csr_rows(int n, F&& f) {
 }
 
 // sum over the row of A[row, j] * xf(j), reduced over the lane group (valid in every lane)
+constexpr int CSR_UNROLL = 4;
 template <class XF>
 __device__ __forceinline__ cx<double> csr_row(const CsrView& A, int row, int l, bool valid, XF&& xf) {
   cx<double> acc = czero<double>();
   if (valid) {
     const long long e1 = A.indptr[row + 1];
-    for (long long e = A.indptr[row] + l; e < e1; e += CSR_LPR) acc = acc + A.data[e] * xf(A.indices[e]);
+    for (long long e = A.indptr[row] + l; e < e1; e += CSR_LPR * CSR_UNROLL) {
+      int j[CSR_UNROLL];
+      cx<double> a[CSR_UNROLL], v[CSR_UNROLL];
+#pragma unroll
+      for (int u = 0; u < CSR_UNROLL; ++u) {
+        const bool in = e + u * CSR_LPR < e1;
+        j[u] = in ? A.indices[e + u * CSR_LPR] : -1;
+        a[u] = in ? A.data[e + u * CSR_LPR] : czero<double>();
+      }
+#pragma unroll
+      for (int u = 0; u < CSR_UNROLL; ++u) v[u] = j[u] >= 0 ? xf(j[u]) : czero<double>();
+#pragma unroll
+      for (int u = 0; u < CSR_UNROLL; ++u)
+        if (j[u] >= 0) acc = acc + a[u] * v[u];
+    }
   }
 #pragma unroll
   for (int o = 1; o < CSR_LPR; o <<= 1) {
@@ -71,12 +94,9 @@ __global__ void __launch_bounds__(CSR_NT) k_csr_spmv(CsrView A, const cx<double>
 }
 
 struct CsrBufs {
-  cx<double>* P0;
-  cx<double>* P1;
-  cx<double>* V0;
-  cx<double>* V1;
+  cx<double>* p;
+  cx<double>* v;
   cx<double>* r;
-  cx<double>* s;
   cx<double>* t;
   cx<double>* x;
   const cx<double>* b;
@@ -93,7 +113,7 @@ __device__ __forceinline__ void csr_pass(const CsrView& A, RedBuf rb, Body&& bod
   if (grid_reduce<CSR_NT, NRED>(acc, rb, shred, sums)) fin(sums);
 }
 
-// Start: r = b - A x (x = 0 unless a guess is given), rho = (rh, r), |r|^2, |b|^2.
+// Start: r = b - A x (x = 0 unless a guess is given), p = r, rho = (rh, r), |r|^2, |b|^2.
 __global__ void __launch_bounds__(CSR_NT) k_csr_init(CsrView A, CsrBufs B, int guess, unsigned seed, KState* st,
                                                     RedBuf rb) {
   csr_pass<4>(A, rb, [&](int row, int l, bool valid, double* acc) {
@@ -103,14 +123,9 @@ __global__ void __launch_bounds__(CSR_NT) k_csr_init(CsrView A, CsrBufs B, int g
       const cx<double> bv = B.b[row];
       const cx<double> r = bv - ax;
       B.r[row] = r;
-      B.P0[row] = czero<double>();
-      B.V0[row] = czero<double>();
-      B.P1[row] = czero<double>();
-      B.V1[row] = czero<double>();
+      B.p[row] = r;
       if (!guess) B.x[row] = czero<double>();
-      const cx<double> h = shadow<double>(row, seed);
-      acc[0] += h.re * r.re + h.im * r.im;
-      acc[1] += h.re * r.im - h.im * r.re;
+      acc_cdot<double>(acc, shadow<double>(row, seed), r);
       acc[2] += cabs2(r);
       acc[3] += cabs2(bv);
     }
@@ -131,25 +146,14 @@ __global__ void __launch_bounds__(CSR_NT) k_csr_init(CsrView A, CsrBufs B, int g
   });
 }
 
-__global__ void __launch_bounds__(CSR_NT) k_csr_a(CsrView A, CsrBufs B, unsigned seed, KState* st, RedBuf rb) {
+__global__ void __launch_bounds__(CSR_NT, 3) k_csr_a(CsrView A, CsrBufs B, unsigned seed, KState* st, RedBuf rb) {
+  pass_begin();
   if (ld_status(st) != ST_RUNNING) return;
-  const bool odd = (__ldcg(&st->iter) & 1) != 0;
-  const cx<double>* Po = odd ? B.P1 : B.P0;
-  const cx<double>* Vo = odd ? B.V1 : B.V0;
-  cx<double>* Pn = odd ? B.P0 : B.P1;
-  cx<double>* Vn = odd ? B.V0 : B.V1;
-  const dcx bd = ld_dcx(&st->beta), od = ld_dcx(&st->omega);
-  const cx<double> beta = from_d<double>(bd), mbo = from_d<double>(dmul(bd, {-od.re, -od.im}));
-  // p = r + beta p_old - beta omega v_old
-  auto pnew = [&](int j) { return caxpy(mbo, Vo[j], caxpy(beta, Po[j], B.r[j])); };
   csr_pass<2>(A, rb, [&](int row, int l, bool valid, double* acc) {
-    const cx<double> v = csr_row(A, row, l, valid, pnew);
+    const cx<double> v = csr_row(A, row, l, valid, [&](int j) { return B.p[j]; });
     if (valid && l == 0) {
-      Pn[row] = pnew(row);
-      Vn[row] = v;
-      const cx<double> h = shadow<double>(row, seed);
-      acc[0] += h.re * v.re + h.im * v.im;
-      acc[1] += h.re * v.im - h.im * v.re;
+      B.v[row] = v;
+      acc_cdot<double>(acc, shadow<double>(row, seed), v);
     }
   }, [&](const double* s) {
     const dcx sigma = {s[0], s[1]};
@@ -159,73 +163,76 @@ __global__ void __launch_bounds__(CSR_NT) k_csr_a(CsrView A, CsrBufs B, unsigned
   });
 }
 
-__global__ void __launch_bounds__(CSR_NT) k_csr_b(CsrView A, CsrBufs B, KState* st, RedBuf rb) {
+__global__ void __launch_bounds__(CSR_NT, 3) k_csr_b(CsrView A, CsrBufs B, unsigned seed, KState* st, RedBuf rb) {
+  pass_begin();
   if (ld_status(st) != ST_RUNNING) return;
-  const bool odd = (__ldcg(&st->iter) & 1) != 0;
-  const cx<double>* V = odd ? B.V0 : B.V1;  // written by this iteration's k_csr_a
   const dcx ad = ld_dcx(&st->alpha);
   const cx<double> malpha = mkc<double>(-ad.re, -ad.im);
-  auto snew = [&](int j) { return caxpy(malpha, V[j], B.r[j]); };
-  csr_pass<4>(A, rb, [&](int row, int l, bool valid, double* acc) {
+  auto snew = [&](int j) { return caxpy(malpha, B.v[j], B.r[j]); };
+  csr_pass<8>(A, rb, [&](int row, int l, bool valid, double* acc) {
     const cx<double> t = csr_row(A, row, l, valid, snew);
     if (valid && l == 0) {
-      const cx<double> s = snew(row);
-      B.s[row] = s;
+      const cx<double> s = snew(row), h = shadow<double>(row, seed);
       B.t[row] = t;
-      acc[0] += t.re * s.re + t.im * s.im;  // (t, s) = conj(t) s
-      acc[1] += t.re * s.im - t.im * s.re;
+      acc_cdot<double>(acc, t, s);
       acc[2] += cabs2(t);
       acc[3] += cabs2(s);
+      acc_cdot<double>(acc + 4, h, s);
+      acc_cdot<double>(acc + 6, h, t);
     }
   }, [&](const double* s) {
-    if (!isfinite(s[0]) || !isfinite(s[1]) || !isfinite(s[2]) || !isfinite(s[3])) {
+    bool ok = true;
+    for (int q = 0; q < 8; ++q) ok = ok && isfinite(s[q]);
+    if (!ok) {
       st->status = ST_NONFINITE;
       return;
     }
+    st->beta = {0.0, 0.0};
     if (s[3] <= st->tol2 || s[2] <= 0.0) {
       // s is small enough (or t vanished): finish this iteration with omega = 0
       st->omega = {0.0, 0.0};
       st->pending = s[3] <= st->tol2 ? 2 : 3;
       return;
     }
-    st->omega = {s[0] / s[2], s[1] / s[2]};
-  });
-}
-
-__global__ void __launch_bounds__(CSR_NT) k_csr_c(CsrView A, CsrBufs B, unsigned seed, KState* st, RedBuf rb) {
-  if (ld_status(st) != ST_RUNNING) return;
-  const bool odd = (__ldcg(&st->iter) & 1) != 0;
-  const cx<double>* P = odd ? B.P0 : B.P1;
-  const cx<double> alpha = from_d<double>(ld_dcx(&st->alpha));
-  const dcx od = ld_dcx(&st->omega);
-  const cx<double> omega = from_d<double>(od), momega = mkc<double>(-od.re, -od.im);
-  csr_pass<3>(A, rb, [&](int row, int l, bool valid, double* acc) {
-    if (valid && l == 0) {
-      const cx<double> s = B.s[row];
-      B.x[row] = caxpy(omega, s, caxpy(alpha, P[row], B.x[row]));
-      const cx<double> r = caxpy(momega, B.t[row], s);
-      B.r[row] = r;
-      const cx<double> h = shadow<double>(row, seed);
-      acc[0] += h.re * r.re + h.im * r.im;
-      acc[1] += h.re * r.im - h.im * r.re;
-      acc[2] += cabs2(r);
-    }
-  }, [&](const double* s) {
-    st->iter += 1;
-    st->rr = s[2];
-    const dcx rho_new = {s[0], s[1]};
-    if (!dfinite(rho_new) || !isfinite(s[2])) { st->status = ST_NONFINITE; return; }
-    if (st->pending == 2 || s[2] <= st->tol2) { st->status = ST_CONVERGED; return; }
-    if (st->pending == 3) { st->status = ST_BREAKDOWN; return; }
-    if (st->iter >= st->maxiter) { st->status = ST_MAXITER; return; }
-    const dcx om = st->omega;
+    const dcx om = {s[0] / s[2], s[1] / s[2]}, w = dmul(om, {s[6], s[7]});
+    const dcx rho_new = {s[4] - w.re, s[5] - w.im};  // (rh, s - omega t)
+    st->omega = om;
     if ((rho_new.re == 0.0 && rho_new.im == 0.0) || (om.re == 0.0 && om.im == 0.0)) {
-      st->status = ST_BREAKDOWN;
+      st->pending = 4;  // a breakdown, unless this iteration converges
       return;
     }
     st->beta = dmul(ddiv(rho_new, st->rho), ddiv(st->alpha, om));
     st->rho = rho_new;
   });
+}
+
+// (elementwise: every lane a row)
+__global__ void __launch_bounds__(CSR_NT) k_csr_c(CsrView A, CsrBufs B, KState* st, RedBuf rb) {
+  pass_begin();
+  if (ld_status(st) != ST_RUNNING) return;
+  const cx<double> alpha = from_d<double>(ld_dcx(&st->alpha)), beta = from_d<double>(ld_dcx(&st->beta));
+  const cx<double> omega = from_d<double>(ld_dcx(&st->omega));
+  const cx<double> malpha = mkc<double>(-alpha.re, -alpha.im), momega = mkc<double>(-omega.re, -omega.im);
+  __shared__ double shred[64];
+  double acc[1] = {0.0};
+  for (long long row = blockIdx.x * (long long)CSR_NT + threadIdx.x; row < A.n; row += (long long)gridDim.x * CSR_NT) {
+    const cx<double> p = B.p[row], v = B.v[row], s = caxpy(malpha, v, B.r[row]);
+    B.x[row] = caxpy(omega, s, caxpy(alpha, p, B.x[row]));
+    const cx<double> r = caxpy(momega, B.t[row], s);
+    B.r[row] = r;
+    B.p[row] = caxpy(beta, caxpy(momega, v, p), r);
+    acc[0] += cabs2(r);
+  }
+  double sums[1];
+  if (grid_reduce<CSR_NT, 1>(acc, rb, shred, sums)) {
+    st->iter += 1;
+    st->rr = sums[0];
+    if (!isfinite(sums[0])) st->status = ST_NONFINITE;
+    else if (st->pending == 2 || sums[0] <= st->tol2) st->status = ST_CONVERGED;
+    else if (st->pending == 3) st->status = ST_BREAKDOWN;
+    else if (st->iter >= st->maxiter) st->status = ST_MAXITER;
+    else if (st->pending == 4) st->status = ST_BREAKDOWN;
+  }
 }
 
 // |b - A x|^2 and |b|^2 (the true residual of the final iterate)

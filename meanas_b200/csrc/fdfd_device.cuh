@@ -146,10 +146,37 @@ struct AccT<float> {
 // ---------------------------------------------------------------- reductions
 // Deterministic grid reduction: every CTA writes its partial sums, the last CTA to
 // finish (atomic ticket) sums them in a fixed order and runs the op's finish().
+//
+// No fence stands between a CTA's partial sums and its ticket: a fence waits for every store
+// in flight, the pass's output vectors among them, and two of them were 2 to 3 us of every
+// pass (COCG stencil pass at 64^3 31.4 -> 29.3 us, CSR elementwise pass 14.2 -> 11.6).  Instead an unwritten partial reads as
+// NO_PARTIAL, the last CTA reads until the value is there, and puts NO_PARTIAL back for the
+// next pass.  The host fills the buffer with it (bytes 0xff) before the first.
 struct RedBuf {
   double* partials;        // [gridDim.x * NRED]
   unsigned int* ticket;    // zero between launches (reset by the last CTA)
 };
+constexpr unsigned long long NO_PARTIAL = ~0ull;  // a NaN that no arithmetic gives
+constexpr int PARTIAL_SPINS = 1 << 22;            // then the sum is NaN
+
+__device__ __forceinline__ void partial_store(double* p, double v) {
+  unsigned long long bits = (unsigned long long)__double_as_longlong(v);
+  if (bits == NO_PARTIAL) bits ^= 1ull;  // still a NaN
+  asm volatile("st.relaxed.gpu.global.u64 [%0], %1;" ::"l"(p), "l"(bits) : "memory");
+}
+__device__ __forceinline__ unsigned long long partial_load(const double* p) {
+  unsigned long long bits;
+  asm volatile("ld.relaxed.gpu.global.u64 %0, [%1];" : "=l"(bits) : "l"(p) : "memory");
+  return bits;
+}
+
+// Start of a pass launched with programmatic stream serialisation: let the next pass's CTAs
+// come up while this one runs, then wait until the pass before has finished and its results
+// are visible.  (No effect in an ordinary launch.)
+__device__ __forceinline__ void pass_begin() {
+  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+  asm volatile("griddepcontrol.wait;" ::: "memory");
+}
 
 // Sum NRED values over the CTA at once: warp trees for all values, one pass through
 // shared memory (sh[warp][r]), then thread r < NRED sums value r over the warps in a
@@ -190,7 +217,7 @@ __device__ __forceinline__ void sum_block_partials(const A* sh, RedBuf rb, size_
     for (int t = lane; t < NT; t += 32) v += (double)sh[r * NT + t];
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) v += __shfl_down_sync(0xffffffffu, v, o);
-    if (lane == 0) rb.partials[part * NRED + r] = v;
+    if (lane == 0) partial_store(&rb.partials[part * NRED + r], v);
   }
 }
 
@@ -203,34 +230,39 @@ __device__ __forceinline__ void write_partial(const A (&acc)[NRED], RedBuf rb, s
 #pragma unroll
   for (int r = 0; r < NRED; ++r) v[r] = (double)acc[r];
   const double s = block_sum_n<NT, NRED>(v, sh);
-  if (tid < NRED) rb.partials[part * NRED + tid] = s;
+  if (tid < NRED) partial_store(&rb.partials[part * NRED + tid], s);
 }
 
-// After every CTA has written its partials: the last CTA to arrive (atomic ticket) sums
-// all `nparts` partials in a fixed order and returns true in its thread 0, which holds
-// the totals in `out`.  The last CTA reads them with independent loads (no per-value
-// passes), so the serial tail after the last CTA's own work is about two L2 round trips.
+// The last CTA to arrive (atomic ticket) sums all `nparts` partials in a fixed order and
+// returns true in its thread 0, which holds the totals in `out`.  The last CTA reads them with
+// independent loads (no per-value passes), so the serial tail after the last CTA's own work
+// is about two L2 round trips.
 template <int NT, int NRED>
 __device__ bool grid_finish(RedBuf rb, unsigned int nparts, double* sh, double* out) {
   const int tid = threadIdx.x + threadIdx.y * blockDim.x;
   __shared__ bool s_last;
-  __threadfence();
-  __syncthreads();
-  if (tid == 0) {
-    __threadfence();  // cumulative: the partials written before the barrier are visible first
-    unsigned int t = atomicAdd(rb.ticket, 1u);
-    s_last = (t == gridDim.x - 1);
-  }
+  if (tid == 0) s_last = atomicAdd(rb.ticket, 1u) == gridDim.x - 1;
   __syncthreads();
   if (!s_last) return false;
-  __threadfence();
   double s[NRED];
 #pragma unroll
   for (int r = 0; r < NRED; ++r) s[r] = 0.0;
-#pragma unroll 4
   for (unsigned int b = tid; b < nparts; b += NT) {
+    double* const p = rb.partials + (size_t)b * NRED;
+    unsigned long long v[NRED];
+    bool all = false;
+    for (int spin = 0; spin < PARTIAL_SPINS && !all; ++spin) {
+      all = true;
 #pragma unroll
-    for (int r = 0; r < NRED; ++r) s[r] += __ldcg(&rb.partials[(size_t)b * NRED + r]);
+      for (int r = 0; r < NRED; ++r) v[r] = partial_load(p + r);
+#pragma unroll
+      for (int r = 0; r < NRED; ++r) all = all && v[r] != NO_PARTIAL;
+    }
+#pragma unroll
+    for (int r = 0; r < NRED; ++r) {
+      s[r] += __longlong_as_double((long long)v[r]);
+      p[r] = __longlong_as_double((long long)NO_PARTIAL);
+    }
   }
   const double tot = block_sum_n<NT, NRED>(s, sh);
   __syncthreads();  // sh reads of block_sum_n done

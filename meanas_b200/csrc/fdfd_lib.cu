@@ -278,6 +278,23 @@ static int ensure_smem(K kern, size_t bytes) {
   return 0;
 }
 
+// Launch a pass whose kernel calls pass_begin(): its CTAs may come up before the pass in
+// front of it on the stream has finished.
+template <class... KArgs, class... Args>
+static cudaError_t launch_pass(void (*kern)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t s, Args... args) {
+  cudaLaunchConfig_t cfg{};
+  cfg.gridDim = grid;
+  cfg.blockDim = block;
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = s;
+  cudaLaunchAttribute at{};
+  at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  at.val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = &at;
+  cfg.numAttrs = 1;
+  return cudaLaunchKernelEx(&cfg, kern, KArgs(args)...);
+}
+
 template <typename R, bool FLAT, bool MAT, class Op>
 static int launch_stencil_as(fdfd_plan* P, const Tiling& t, const Geo<R>& g, const Op& op, RedBuf rb, cudaStream_t s) {
   constexpr int TZ = FLAT ? 1 : TZ3, TY = FLAT ? FLAT_TY : TY3;
@@ -739,6 +756,14 @@ extern "C" int fdfd_residual_workspace_bytes(const fdfd_plan* P, size_t* bytes) 
   return 0;
 }
 
+// A reduction buffer before its first pass: ticket zero, `n` partial sums unwritten.  (Every
+// pass leaves it like that again.)
+static int red_init(RedBuf rb, size_t n, cudaStream_t s) {
+  CK(cudaMemsetAsync(rb.ticket, 0, sizeof(unsigned int), s));
+  CK(cudaMemsetAsync(rb.partials, 0xff, n * sizeof(double), s));
+  return 0;
+}
+
 static int residual_into(fdfd_plan* P, const void* E, const void* J, int adjoint, double* d_out, RedBuf rb,
                          cudaStream_t s) {
   OpResidual<double> o{(const cx<double>*)E, (const cx<double>*)J, P->om_re, P->om_im, adjoint, P->g64, d_out};
@@ -758,7 +783,7 @@ extern "C" int fdfd_residual(fdfd_plan* P, const void* E, const void* J, double 
   double* d_out = (double*)(base + 256);
   RedBuf rb{(double*)(base + 512), ticket};
   P->launches = 0;
-  CK(cudaMemsetAsync(ticket, 0, sizeof(unsigned int), s));
+  TRY(red_init(rb, (size_t)stencil_parts(P, make_tiling(P, 0)) * OpResidual<double>::NRED, s));
   TRY(residual_into(P, E, J, 0, d_out, rb, s));
   CK(cudaMemcpyAsync(P->h_state, d_out, 4 * sizeof(double), cudaMemcpyDeviceToHost, s));
   CK(cudaStreamSynchronize(s));
@@ -1137,7 +1162,7 @@ extern "C" int fdfd_solve(fdfd_plan* P, const fdfd_solve_opts* o, const void* J,
 
   KState h = make_state(o, c.crit, maxiter, o->history);
   *P->h_state = h;
-  CK(cudaMemsetAsync(ticket, 0, sizeof(unsigned int), s));
+  TRY(red_init(c.rb, (size_t)max_blocks(P) * 8, s));
   CK(cudaMemsetAsync(c.scratch, 0, sizeof(ResidentScratch), s));
   CK(cudaMemcpyAsync(c.st, P->h_state, sizeof(KState), cudaMemcpyHostToDevice, s));
   // right-hand side (and guess) in the solve space; E holds the iterate
@@ -1372,22 +1397,28 @@ static int csr_view(const fdfd_csr_desc* d, CsrView* v, const char* who) {
   return 0;
 }
 
-// CTAs for the CSR kernels: enough rows per CTA step to cover n, at most 8 per SM
-static unsigned csr_blocks(int n) {
+// CTAs for a CSR kernel: enough for `per_cta` rows each, at most its resident slots (a second,
+// partial wave of CTAs costs a kernel of this length more than a longer loop).
+static unsigned csr_blocks(int n, int per_cta, int occ) {
   int dev = 0, nsm = 148;
   cudaGetDevice(&dev);
   cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev);
-  const long long rows_per_cta = CSR_NT / CSR_LPR;
-  const long long need = (n + rows_per_cta - 1) / rows_per_cta;
-  return (unsigned)std::max(1LL, std::min(need, 8LL * nsm));
+  const long long need = ((long long)n + per_cta - 1) / per_cta;
+  return (unsigned)std::max(1LL, std::min(need, (long long)occ * nsm));
 }
+static constexpr int CSR_ROWS = CSR_NT / CSR_LPR;  // rows per CTA step
+#define CSR_GRID(kern, n, per_cta)                      \
+  [](int n_) {                                          \
+    static const int occ = occupancy(kern, CSR_NT);     \
+    return csr_blocks(n_, per_cta, occ);                \
+  }(n)
 
 extern "C" int fdfd_csr_spmv(const fdfd_csr_desc* d, const void* x, void* y, void* stream) {
   CsrView A;
   TRY(csr_view(d, &A, "fdfd_csr_spmv"));
   if (!x || !y) return set_err(FDFD_ERR_ARG, "fdfd_csr_spmv: NULL vector");
   if (x == y) return set_err(FDFD_ERR_ARG, "fdfd_csr_spmv: y must not alias x");
-  k_csr_spmv<<<csr_blocks(A.n), CSR_NT, 0, (cudaStream_t)stream>>>(A, (const cx<double>*)x, (cx<double>*)y);
+  k_csr_spmv<<<CSR_GRID(k_csr_spmv, A.n, CSR_ROWS), CSR_NT, 0, (cudaStream_t)stream>>>(A, (const cx<double>*)x, (cx<double>*)y);
   CKL();
   return 0;
 }
@@ -1408,7 +1439,7 @@ static CsrLayout csr_layout(int n) {
   L.ticket = take(sizeof(unsigned));
   L.partials = take(sizeof(double) * 8 * (size_t)8 * 2048);  // up to 8 sums x 16k CTAs
   L.res = take(2 * sizeof(double));
-  L.vec = take(7 * 16 * (size_t)n);
+  L.vec = take(4 * 16 * (size_t)n);
   L.total = off;
   return L;
 }
@@ -1437,7 +1468,6 @@ extern "C" int fdfd_csr_solve(const fdfd_csr_desc* d, const fdfd_solve_opts* o, 
   const size_t vb = 16 * (size_t)A.n;
   cx<double>* V = (cx<double>*)(w + L.vec);
   CsrBufs B{V, (cx<double>*)((char*)V + vb), (cx<double>*)((char*)V + 2 * vb), (cx<double>*)((char*)V + 3 * vb),
-            (cx<double>*)((char*)V + 4 * vb), (cx<double>*)((char*)V + 5 * vb), (cx<double>*)((char*)V + 6 * vb),
             (cx<double>*)x, (const cx<double>*)b};
   KState h{};
   h.rtol = o->rtol;
@@ -1445,10 +1475,12 @@ extern "C" int fdfd_csr_solve(const fdfd_csr_desc* d, const fdfd_solve_opts* o, 
   h.maxiter = o->maxiter > 0 ? o->maxiter : 10 * A.n;
   h.status = ST_RUNNING;
   CK(cudaMemcpyAsync(st, &h, sizeof(KState), cudaMemcpyHostToDevice, s));
-  CK(cudaMemsetAsync(rb.ticket, 0, sizeof(unsigned), s));
-  const unsigned grid = csr_blocks(A.n);
+  const unsigned grid = CSR_GRID(k_csr_init, A.n, CSR_ROWS), grid_a = CSR_GRID(k_csr_a, A.n, CSR_ROWS);
+  const unsigned grid_b = CSR_GRID(k_csr_b, A.n, CSR_ROWS), grid_c = CSR_GRID(k_csr_c, A.n, CSR_NT);
+  const unsigned grid_r = CSR_GRID(k_csr_residual, A.n, CSR_ROWS);
   const unsigned seed = 0x5eed5eedU;
   int launches = 0;
+  TRY(red_init(rb, (size_t)std::max({grid, grid_a, grid_b, grid_c, grid_r}) * 8, s));
   k_csr_init<<<grid, CSR_NT, 0, s>>>(A, B, o->has_guess != 0, seed, st, rb);
   CKL();
   ++launches;
@@ -1462,16 +1494,15 @@ extern "C" int fdfd_csr_solve(const fdfd_csr_desc* d, const fdfd_solve_opts* o, 
     status = head[3];
     if (status != ST_RUNNING || iters >= h.maxiter) break;
     for (int it = 0; it < chunk; ++it) {
-      k_csr_a<<<grid, CSR_NT, 0, s>>>(A, B, seed, st, rb);
-      k_csr_b<<<grid, CSR_NT, 0, s>>>(A, B, st, rb);
-      k_csr_c<<<grid, CSR_NT, 0, s>>>(A, B, seed, st, rb);
-      CKL();
+      CK(launch_pass(k_csr_a, grid_a, CSR_NT, 0, s, A, B, seed, st, rb));
+      CK(launch_pass(k_csr_b, grid_b, CSR_NT, 0, s, A, B, seed, st, rb));
+      CK(launch_pass(k_csr_c, grid_c, CSR_NT, 0, s, A, B, st, rb));
       launches += 3;
     }
   }
   if (status == ST_RUNNING) status = ST_MAXITER;
   double* res = (double*)(w + L.res);
-  k_csr_residual<<<grid, CSR_NT, 0, s>>>(A, (const cx<double>*)x, (const cx<double>*)b, res, rb);
+  k_csr_residual<<<grid_r, CSR_NT, 0, s>>>(A, (const cx<double>*)x, (const cx<double>*)b, res, rb);
   CKL();
   ++launches;
   double hr[2];
@@ -1648,8 +1679,7 @@ extern "C" int fdfd_residual_static(fdfd_plan* P, const void* E, const void* J, 
   double* d_out = (double*)(b + 256);
   RedBuf rb{(double*)(b + 512), ticket};
   P->launches = 0;
-  // the ticket must start at zero; the partials and sums are fully rewritten
-  CK(cudaMemsetAsync(ticket, 0, sizeof(unsigned int), s));
+  TRY(red_init(rb, (size_t)parts * OpResidual<double>::NRED, s));
   TRY(residual_into(P, E, J, 0, d_out, rb, s));
   CK(cudaMemcpyAsync(P->h_state, d_out, 4 * sizeof(double), cudaMemcpyDeviceToHost, s));
   CK(cudaStreamSynchronize(s));
