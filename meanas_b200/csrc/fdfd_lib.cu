@@ -136,6 +136,7 @@ struct fdfd_plan {
   int nsm;
   int rb_shift;            // reductions over blocks of 2^rb_shift x planes (a grid property)
   int xc_override[2];
+  int xc128;               // x planes per CTA of the complex128 passes (default_xchunk)
   Geo<double> g64;
   Geo<float> g32;
   cudaStream_t cap;        // private stream for graph capture
@@ -207,6 +208,45 @@ static constexpr int TZ3 = 32, TY3 = 8;
 
 static size_t align256(size_t v) { return (v + 255) & ~(size_t)255; }
 
+// x planes per CTA for the complex128 passes: the choice (whole reduction blocks) whose CTAs,
+// taken in order by the resident slots, finish first.  A CTA costs its planes and a prologue
+// of about 2.5; the last chunk may be short.  The results do not depend on it (the sums run
+// over a fixed partition).  COCG stencil pass, the earlier rule of about eight CTAs per SM /
+// this one: 160x160x128 (16 / 48 planes) 208 / 198 us, 128^3 (8 / 32) 153 / 135, 121x97x109 with
+// masks (8 / 24) 153 / 143, flat 700x613 (4 / 8) 48 / 42.  (Complex64 passes, throughput-bound at three or four CTAs per SM,
+// do not follow this model and keep that rule.)
+static int default_xchunk(const fdfd_plan* P) {
+  const int TZ = P->flat ? 1 : TZ3, TY = P->flat ? FLAT_TY : TY3, rbp = 1 << P->rb_shift;
+  const long long tiles = (long long)((P->Z + TZ - 1) / TZ) * ((P->Y + TY - 1) / TY), slots = 2LL * P->nsm;
+  int best = rbp;
+  double best_t = -1.0;
+  for (int xc = rbp; xc <= XC_MAX; xc += rbp) {
+    const double full = xc + 2.5, part = P->X % xc + 2.5;
+    const long long nf = tiles * (P->X / xc);
+    // full chunks first: `busy` slots end with the last round, the others one round earlier
+    const long long rounds = (nf + slots - 1) / slots, busy = nf - std::max(0LL, rounds - 1) * slots;
+    double t = rounds * full;
+    if (P->X % xc) {
+      // then the short ones, on whichever slots are free first
+      double early = std::max(0.0, (rounds - 1) * full), late = rounds * full;
+      long long ne = slots - busy, left = tiles;
+      while (left > 0) {
+        const bool on_early = ne > 0 && early <= late;
+        const long long n = std::min(left, on_early ? ne : std::max(1LL, busy));
+        (on_early ? early : late) += part;
+        left -= n;
+        t = std::max(t, on_early ? early : late);
+      }
+    }
+    if (best_t < 0 || t < best_t) {
+      best_t = t;
+      best = xc;
+    }
+    if (xc >= P->X) break;
+  }
+  return best;
+}
+
 static Tiling make_tiling(const fdfd_plan* P, int precision) {
   Tiling t;
   const int TZ = P->flat ? 1 : TZ3, TY = P->flat ? FLAT_TY : TY3;
@@ -214,6 +254,7 @@ static Tiling make_tiling(const fdfd_plan* P, int precision) {
   t.nty = (P->Y + TY - 1) / TY;
   const long long tiles = (long long)t.ntz * t.nty;
   int xc = P->xc_override[precision];
+  if (xc <= 0 && precision == 0) xc = P->xc128;
   if (xc <= 0) {
     // aim for about 8 CTAs per SM in total (two waves at 4 resident CTAs per SM)
     const long long target = 8LL * P->nsm;
@@ -612,6 +653,7 @@ extern "C" int fdfd_plan_create(const fdfd_grid_desc* d, void* ws, size_t ws_byt
       cudaMallocHost((void**)&P->h_state, sizeof(KState)) != cudaSuccess)
     return cleanup(set_err(FDFD_ERR_CUDA, "plan: stream/event/pinned allocation failed"));
 
+  P->xc128 = default_xchunk(P);
   P->ws = (char*)ws;
   P->has_mu = d->mu != nullptr;
   P->has_mask = (d->pec != nullptr) || (d->pmc != nullptr);
