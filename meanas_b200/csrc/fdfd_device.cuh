@@ -324,7 +324,7 @@ __device__ __forceinline__ void run_finish(const Op& o, const double* sums) {
 //   bool skip() const;             uniform early exit (solver stopped)
 //   void prepare();                read scalars once per thread
 //   const cx<R>* box_src(int b) const;               null = zeros
-//   const cx<R>* own_src(int o) const;               null = zeros
+//   const cx<R>* own_src(int o) const;               null = not read (values undefined)
 //   cx<R> make_u(const cx<R>* v, int idx, int c) const;   input field from raw values
 //   void convert_own(const cx<R>* v, const cx<R>* ov, int idx, int c, cx<R> u, A* acc) const;
 //        own cells of the CTA's planes, when their inputs land: outputs that do not need
@@ -526,8 +526,7 @@ __device__ __forceinline__ void stencil_unit(const Geo<R>& g, const Op& o, RedBu
 #pragma unroll
       for (int c = 0; c < 3; ++c) {
         cx<R>* dst = Sown + (oi * 3 + c) * NT + tid;
-        if (src) cp_async_cx<R>(dst, src + c * N + base + off0);
-        else *dst = czero<R>();
+        if (src) cp_async_cx<R>(dst, src + c * N + base + off0);  // (null: not read)
       }
     }
     cp_async_commit();

@@ -1060,12 +1060,20 @@ static int cocg_loop(SolveCtx& c, cx<double>* r, cx<double>* q, cx<double>* P0, 
   RedBuf rb = c.rb;
   const int chunk = c.chunk;
   cx<double>* x = c.x;
+  // x updates two at a time (see OpCocgA): from a million cells on the five vectors of a pass
+  // (240 MB) no longer fit L2
+  const bool two = P->N >= (1LL << 20) && !P->has_mu && !P->has_mask;
   auto enqueue = [&](cudaStream_t ss) -> int {
     for (int it = 0; it < chunk; ++it) {
       {
         ProfScope ps(P, 0, ss);
-        OpCocgA<double> a{r, P0, P1, x, q, N, st};
-        TRY(launch_stencil<double>(P, P->g64, 0, a, rb, ss));
+        if (two) {
+          OpCocgA<double, true> a{r, P0, P1, x, q, N, st};
+          TRY(launch_stencil<double>(P, P->g64, 0, a, rb, ss));
+        } else {
+          OpCocgA<double, false> a{r, P0, P1, x, q, N, st};
+          TRY(launch_stencil<double>(P, P->g64, 0, a, rb, ss));
+        }
       }
       {
         ProfScope ps(P, 1, ss);

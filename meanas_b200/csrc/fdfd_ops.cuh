@@ -39,6 +39,7 @@ constexpr double BREAKDOWN_RATIO = 1e-14;
 // FP64 scalar state of one Krylov sequence (device memory).
 struct KState {
   dcx rho, sigma, alpha, beta, omega;
+  dcx alpha_prev;  // COCG: the step before alpha's, while its x update is owed too
   double rr;       // |r|^2 (recurrence residual)
   double rr_pc;    // sum |W| |r|^2
   double rr_w2;    // sum |W|^2 |r|^2
@@ -51,7 +52,7 @@ struct KState {
   double extra[4];
   int crit;        // 0: monitor rr, 1: monitor rr_pc, 2: monitor rr_w2
   int iter, maxiter, status;
-  int pending;     // an x update is still owed (deferred update)
+  int pending;     // x updates still owed (deferred; the codes are the solvers')
   int stall_limit; // BiCGSTAB: stop (ST_BREAKDOWN) after this many iterations without a new
                    // best residual (0 = never)
   double best_rr;  // BiCGSTAB: best recurrence residual so far, and its iteration
@@ -334,10 +335,18 @@ struct OpCocgInit {
   }
 };
 
-// p = r + beta p_old ; x += alpha p_old (deferred) ; q = A0 p ; sigma = p^T W q
-template <typename R>
+// p = r + beta p_old ; q = A0 p ; sigma = p^T W q, and the x updates of the steps before.
+// TWO = false: x += alpha p_old in every pass.  TWO = true: two updates in every second pass;
+// p of the step before is at hand and p of the one before that is what p_new overwrites, so
+// they share one read and write of x (312 -> 288 bytes per cell on average).  It wins where
+// the vectors come from HBM and costs registers and shared memory otherwise; stencil pass,
+// TWO = false / true: 160x160x128 198 / 192 us, 128^3 135 / 129; 64^3 29.4 / 31.6, flat 700x613
+// 42 / 44, with mu and masks at 121x97x109 (where it spills) 143 / 166.
+// pending: 1 = x owes alpha p_old, 2 = x also owes alpha_prev times the p before, 3 = it owes
+// only that one (the last step was discarded).
+template <typename R, bool TWO>
 struct OpCocgA {
-  static constexpr int NB = 2, NO = 1, NRED = 2;
+  static constexpr int NB = 2, NO = TWO ? 2 : 1, NRED = 2;
   static constexpr bool NEEDS_W = true;
   const cx<R>* r;
   cx<R>* P0;
@@ -349,7 +358,7 @@ struct OpCocgA {
   // per-thread
   const cx<R>* p_old;
   cx<R>* p_new;
-  cx<R> beta, alpha;
+  cx<R> beta, alpha, alpha_prev;
   bool upd;
   struct Pre {};
   __device__ bool skip() const { return ld_status(st) != ST_RUNNING; }
@@ -359,16 +368,17 @@ struct OpCocgA {
     p_new = (k & 1) ? P0 : P1;
     beta = from_d<R>(ld_dcx(&st->beta));
     alpha = from_d<R>(ld_dcx(&st->alpha));
-    upd = __ldcg(&st->pending) != 0;
+    if (TWO) alpha_prev = from_d<R>(ld_dcx(&st->alpha_prev));
+    upd = __ldcg(&st->pending) >= (TWO ? 2 : 1);
   }
   __device__ const cx<R>* box_src(int bi) const { return bi == 0 ? r : p_old; }
-  __device__ const cx<R>* own_src(int) const { return upd ? x : nullptr; }
+  __device__ const cx<R>* own_src(int oi) const { return upd ? (oi == 0 ? x : p_new) : nullptr; }
   __device__ void pre(int, Pre&) const {}
-  // v = [r, p_old], ov = [x]
+  // v = [r, p_old], ov = [x, the p before p_old]
   __device__ cx<R> make_u(const cx<R>* v, int, int) const { return caxpy(beta, v[1], v[0]); }
   __device__ void convert_own(const cx<R>* v, const cx<R>* ov, int idx, int, cx<R> u, acc_t<R>*) const {
     p_new[idx] = u;
-    if (upd) x[idx] = caxpy(alpha, v[1], ov[0]);
+    if (upd) x[idx] = caxpy(alpha, v[1], TWO ? caxpy(alpha_prev, ov[NO - 1], ov[0]) : ov[0]);
   }
   __device__ void own(int cell, int, int, int, const cx<R> u[3], const cx<R> y[3], const cx<R> W[3],
                       const R*, const Pre&, acc_t<R>* acc) const {
@@ -383,7 +393,7 @@ struct OpCocgA {
   __device__ void finish(const double* s) const {
     const dcx sigma = {s[0], s[1]};
     st->sigma = sigma;
-    st->pending = 0;
+    if (!TWO || st->pending == 2) st->pending = 0;
     if (!dfinite(sigma)) {
       st->status = ST_NONFINITE;
       return;
@@ -394,6 +404,7 @@ struct OpCocgA {
       st->status = ST_BREAKDOWN;
       return;
     }
+    st->alpha_prev = st->alpha;
     st->alpha = ddiv(st->rho, sigma);
   }
 };
@@ -436,10 +447,11 @@ struct OpCocgB {
     st->rr_w2 = s[4];
     st->iter += 1;
     const bool ok = dfinite(rho_new);
-    st->pending = ok ? 1 : 0;
+    const int owed = st->pending;  // 0 or 1: the step before is owed
+    st->pending = ok ? owed + 1 : 3 * owed;
     // a near-zero p^T W q shows up as a residual explosion: the step is discarded
     if (ok && s[3] > 1e16 * prev_pc) {
-      st->pending = 0;
+      st->pending = 3 * owed;
       st->status = ST_BREAKDOWN;
       return;
     }
@@ -458,7 +470,7 @@ struct OpCocgB {
   }
 };
 
-// x += alpha * p_last if an update is owed (after the loop stops).
+// The x updates still owed after the loop stops (the codes of OpCocgA).
 template <typename R>
 struct OpCocgFinal {
   static constexpr int NRED = 0;
@@ -469,21 +481,27 @@ struct OpCocgFinal {
   int N;
   KState* st;
   const cx<R>* p;
-  cx<R> alpha;
-  bool upd;
-  __device__ bool skip() const { return false; }
+  const cx<R>* p_before;
+  cx<R> alpha, alpha_prev;
+  int owed;
+  __device__ bool skip() const { return __ldcg(&st->pending) == 0; }
   __device__ void prepare() {
     const int k = __ldcg(&st->iter);
+    owed = __ldcg(&st->pending);
+    // a discarded step has counted: its p is the newer buffer all the same
     p = (k & 1) ? P1 : P0;
+    p_before = (k & 1) ? P0 : P1;
     alpha = from_d<R>(ld_dcx(&st->alpha));
-    upd = __ldcg(&st->pending) != 0;
+    alpha_prev = from_d<R>(ld_dcx(&st->alpha_prev));
   }
   __device__ void point(int cell, int, int, int, const cx<R>*, const R*, acc_t<R>*) const {
-    if (!upd) return;
 #pragma unroll
     for (int c = 0; c < 3; ++c) {
       const int idx = c * N + cell;
-      x[idx] = caxpy(alpha, p[idx], x[idx]);
+      cx<R> v = x[idx];
+      if (owed != 1) v = caxpy(alpha_prev, p_before[idx], v);
+      if (owed != 3) v = caxpy(alpha, p[idx], v);
+      x[idx] = v;
     }
   }
   __device__ void finish(const double*) const {}

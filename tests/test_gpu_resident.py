@@ -135,3 +135,35 @@ def test_mixed_solution_matches_cocg(cuda, shape):
     assert info.converged and ref.converged and info.residual <= 1e-11 * 1.01
     # both residuals are at 1e-11; the lossy operator's condition number is below 1e4
     assert float((E - Er).norm()) <= 1e-7 * float(Er.norm())
+
+
+@pytest.mark.parametrize('steps', [0, 1, 2, 3, 4, 5])
+@pytest.mark.parametrize('shape', [(9, 8, 33), (12, 70, 1)], ids=str)
+def test_owed_updates_are_made_wherever_the_loop_stops(cuda, shape, steps):
+    """The two-launch form owes its x updates for a pass: after any number of iterations the
+    field equals the resident form's, which makes them at once (few steps: only the order
+    of the sums differs, 1e-16 times a cancellation below 1e3)."""
+    from meanas_b200.operators import GridOperator
+    p, J, guess = _problem(shape, False, seed=3)
+    op = GridOperator(**p, device=cuda, fp32=False)
+    kw = dict(rtol=1e-13, criterion='true', maxiter=steps, E_guess=guess)
+    E, info = op.solve(J, **kw)
+    Er, ref = op.solve(J, profile=True, **kw)
+    assert info.iterations == ref.iterations == steps
+    assert float((E - Er).norm()) <= 1e-12 * float(Er.norm())
+
+
+@pytest.mark.parametrize('steps', [1, 2, 3, 4, 5])
+def test_updates_two_at_a_time(cuda, steps):
+    """From a million cells on, x is updated in every second pass; an all-zero
+    conductor mask selects the update in every pass on the same problem: the same field."""
+    from meanas_b200.operators import GridOperator
+    p, J, _ = _problem((129, 64, 128), False, seed=3)
+    J = numpy.where(numpy.arange(J.size) % 977 == 500, J, 0)
+    op = GridOperator(**p, device=cuda, fp32=False)
+    E, info = op.solve(J, rtol=1e-13, criterion='true', maxiter=steps)
+    p['pmc'] = numpy.zeros(J.size)
+    ref_op = GridOperator(**p, device=cuda, fp32=False)
+    Er, ref = ref_op.solve(J, rtol=1e-13, criterion='true', maxiter=steps)
+    assert info.iterations == ref.iterations == steps
+    assert float((E - Er).norm()) <= 1e-13 * float(Er.norm())
