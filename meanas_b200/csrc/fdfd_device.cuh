@@ -78,6 +78,26 @@ __device__ __forceinline__ bool dfinite(dcx a) { return isfinite(a.re) && isfini
 template <typename R>
 __device__ __forceinline__ cx<R> from_d(dcx a) { return mkc<R>((R)a.re, (R)a.im); }
 
+// Quotient of n < 2^31 by a fixed divisor, by a multiplication and a shift (Granlund and
+// Montgomery's round-up method with a 32-bit multiplier and the carry added back).
+struct FastDiv {
+  unsigned mul, shift, d;
+  void init(unsigned div) {
+    d = div;
+    shift = 0;
+    while ((1ull << shift) < div) ++shift;
+    mul = (unsigned)(((1ull << 32) * ((1ull << shift) - div)) / div + 1);
+  }
+  __host__ __device__ __forceinline__ unsigned operator()(unsigned n) const {
+#ifdef __CUDA_ARCH__
+    const unsigned t = __umulhi(n, mul);
+#else
+    const unsigned t = (unsigned)(((unsigned long long)n * mul) >> 32);
+#endif
+    return (t + n) >> shift;  // t + n < 2^32: n < 2^31 and t <= n
+  }
+};
+
 // ---------------------------------------------------------------- grid description
 // Mask byte per cell: bits 0..2 = PEC on the x/y/z E component, bits 3..5 = PMC on
 // the x/y/z H component (meanas/fdfd/operators.py:79-87: any nonzero = conductor).
@@ -794,37 +814,37 @@ __global__ void __launch_bounds__(TZ * TY, MINB) k_stencil(const Geo<R> g, Op op
 }
 
 // ---------------------------------------------------------------- pointwise engine
-// Own cells only, no stencil.  Work units are (x plane, y/z tile) pairs, tiles fastest;
-// the grid is sized to the GPU's resident CTA slots and CTA b takes units b, b + grid,
-// b + 2 grid, ...  The assignment is fixed (the reductions stay deterministic) and every
-// SM streams to the end instead of idling through a partial last wave.
+// Own cells only, no stencil.  Cells go to threads by number, so every lane works on any
+// shape (32 x 8 tiles left a fifth of them idle at 121x97x109); the grid is sized to the GPU's
+// resident CTA slots and CTA b takes runs of NT cells b, b + grid, b + 2 grid, ...  The
+// assignment is fixed (the reductions stay deterministic) and every SM streams to the end
+// instead of idling through a partial last wave.  COCG pointwise pass, tiles / by number:
+// 121x97x109 53.7 / 48.0 us, 160x160x128 94.8 / 92.1 (5.1 TB/s: HBM with two reads per write), flat
+// 700x613 25.3 / 23.6.  Two cells per turn (92 -> 100 us) or more CTAs than registers allow
+// (97 to 135) are slower.
 //   void point(int cell, int i, int j, int k, const cx<R> W[3], const R aW[3], A* acc);
-template <typename R, int TZ, int TY, class Op>
-__device__ __forceinline__ void point_units(const Geo<R>& g, const Op& o, typename AccT<R>::type* acc) {
-  const int tz = threadIdx.x, ty = threadIdx.y;
-  const int ntiles = g.ntz * g.nty;
-  const int units = ntiles * g.X;
-  const int YZ = g.Y * g.Z;
-  for (int u = blockIdx.x; u < units; u += gridDim.x) {
-    const int i = u / ntiles, t = u - i * ntiles;
-    const int tyb = t / g.ntz, tzb = t - tyb * g.ntz;
-    const int j = tyb * TY + ty, k = tzb * TZ + tz;
-    if (j < g.Y && k < g.Z) {
-      cx<R> W[3];
-      R aW[3];
-      if (Op::NEEDS_W) {
-        WeightYZ<R> wyz;
-        wyz.init(g, j, k);
-        wyz.at(g.dxe[0][i], g.dxh[0][i], g.adxe[0][i], g.adxh[0][i], W, aW);
-      }
-      o.point(i * YZ + j * g.Z + k, i, j, k, W, aW, acc);
-    }
+struct CellDiv {  // cell number -> (i, j, k)
+  FastDiv by_z, by_y;
+  int Y, Z;
+  void init(int y, int z) {
+    by_z.init((unsigned)z);
+    by_y.init((unsigned)y);
+    Y = y;
+    Z = z;
   }
-}
+  __device__ __forceinline__ void operator()(int n, int& i, int& j, int& k) const {
+    const int row = (int)by_z((unsigned)n);
+    i = (int)by_y((unsigned)row);
+    j = row - i * Y;
+    k = n - row * Z;
+  }
+};
 
-template <typename R, int TZ, int TY, class Op>
-__global__ void __launch_bounds__(TZ * TY) k_point(const Geo<R> g, Op op, RedBuf rb) {
-  constexpr int NT = TZ * TY;
+constexpr int POINT_NT = 256;
+
+template <typename R, class Op>
+__global__ void __launch_bounds__(POINT_NT) k_point(const Geo<R> g, const CellDiv cd, Op op, RedBuf rb) {
+  constexpr int NT = POINT_NT;
   __shared__ double shred[64];
   if (op.skip()) return;
   Op o = op;
@@ -833,7 +853,18 @@ __global__ void __launch_bounds__(TZ * TY) k_point(const Geo<R> g, Op op, RedBuf
   A acc[Op::NRED > 0 ? Op::NRED : 1];
 #pragma unroll
   for (int r = 0; r < (Op::NRED > 0 ? Op::NRED : 1); ++r) acc[r] = A(0);
-  point_units<R, TZ, TY, Op>(g, o, acc);
+  for (long long n = (long long)blockIdx.x * NT + threadIdx.x; n < g.N; n += (long long)gridDim.x * NT) {
+    int i, j, k;
+    cd((int)n, i, j, k);
+    cx<R> W[3];
+    R aW[3];
+    if (Op::NEEDS_W) {
+      WeightYZ<R> wyz;
+      wyz.init(g, j, k);
+      wyz.at(g.dxe[0][i], g.dxh[0][i], g.adxe[0][i], g.adxh[0][i], W, aW);
+    }
+    o.point((int)n, i, j, k, W, aW, acc);
+  }
   if constexpr (Op::NRED > 0) {
     double sums[Op::NRED];
     // (finish runs on the global state here: a state copy would cost this kernel occupancy)

@@ -28,26 +28,6 @@ struct CpmlFace {
   void* psi_v;
 };
 
-// Quotient of n < 2^31 by a fixed divisor, by a multiplication and a shift (Granlund and
-// Montgomery's round-up method with a 32-bit multiplier and the carry added back).
-struct FastDiv {
-  unsigned mul, shift, d;
-  void init(unsigned div) {
-    d = div;
-    shift = 0;
-    while ((1ull << shift) < div) ++shift;
-    mul = (unsigned)(((1ull << 32) * ((1ull << shift) - div)) / div + 1);
-  }
-  __host__ __device__ __forceinline__ unsigned operator()(unsigned n) const {
-#ifdef __CUDA_ARCH__
-    const unsigned t = __umulhi(n, mul);
-#else
-    const unsigned t = (unsigned)(((unsigned long long)n * mul) >> 32);
-#endif
-    return (t + n) >> shift;  // t + n < 2^32: n < 2^31 and t <= n
-  }
-};
-
 struct FdtdGeo {
   int X, Y, Z;
   // The cells in two lists: those outside the layers along z (all, without layers) and those

@@ -137,6 +137,7 @@ struct fdfd_plan {
   int rb_shift;            // reductions over blocks of 2^rb_shift x planes (a grid property)
   int xc_override[2];
   int xc128;               // x planes per CTA of the complex128 passes (default_xchunk)
+  CellDiv cells;
   Geo<double> g64;
   Geo<float> g32;
   cudaStream_t cap;        // private stream for graph capture
@@ -366,24 +367,16 @@ static int occupancy(K kern, int threads) {
   return n;
 }
 
+// CTAs for a kernel over the plan's cells: one per resident slot (`occ` per SM) at most
+static unsigned point_blocks(const fdfd_plan* P, int occ) {
+  return (unsigned)std::min((P->N + POINT_NT - 1) / POINT_NT, (long long)occ * P->nsm);
+}
+
 template <typename R, class Op>
-static int launch_point(fdfd_plan* P, const Geo<R>& g0, int precision, const Op& op, RedBuf rb,
-                        cudaStream_t s) {
-  const Tiling t = make_tiling(P, precision);
-  const Geo<R> g = geo_with(g0, t);
-  const long long units = (long long)t.ntz * t.nty * P->X;
-  // one CTA per resident slot (occupancy of this kernel, queried once)
-  if (P->flat) {
-    auto kern = k_point<R, 1, FLAT_TY, Op>;
-    static const int occ = occupancy(kern, FLAT_TY);
-    const unsigned grid = (unsigned)std::min(units, (long long)occ * P->nsm);
-    kern<<<grid, dim3(1, FLAT_TY), 0, s>>>(g, op, rb);
-  } else {
-    auto kern = k_point<R, TZ3, TY3, Op>;
-    static const int occ = occupancy(kern, TZ3 * TY3);
-    const unsigned grid = (unsigned)std::min(units, (long long)occ * P->nsm);
-    kern<<<grid, dim3(TZ3, TY3), 0, s>>>(g, op, rb);
-  }
+static int launch_point(fdfd_plan* P, const Geo<R>& g, const Op& op, RedBuf rb, cudaStream_t s) {
+  auto kern = k_point<R, Op>;
+  static const int occ = occupancy(kern, POINT_NT);  // queried once
+  kern<<<point_blocks(P, occ), POINT_NT, 0, s>>>(g, P->cells, op, rb);
   P->launches++;
   CKL();
   return 0;
@@ -654,6 +647,7 @@ extern "C" int fdfd_plan_create(const fdfd_grid_desc* d, void* ws, size_t ws_byt
     return cleanup(set_err(FDFD_ERR_CUDA, "plan: stream/event/pinned allocation failed"));
 
   P->xc128 = default_xchunk(P);
+  P->cells.init(P->Y, P->Z);
   P->ws = (char*)ws;
   P->has_mu = d->mu != nullptr;
   P->has_mask = (d->pec != nullptr) || (d->pmc != nullptr);
@@ -1027,7 +1021,7 @@ static int refine_loop(SolveCtx& c, const Geo<RI>& gi, int prec, BsBufs B, doubl
     }));
     if (!resident) {
       OpBsFinal<RI> fin{B, N, sti};
-      TRY(launch_point<RI>(P, gi, prec, fin, rb, s));
+      TRY(launch_point<RI>(P, gi, fin, rb, s));
     }
     CK(cudaMemcpyAsync(P->h_state, sti, sizeof(KState), cudaMemcpyDeviceToHost, s));
     CK(cudaStreamSynchronize(s));
@@ -1078,7 +1072,7 @@ static int cocg_loop(SolveCtx& c, cx<double>* r, cx<double>* q, cx<double>* P0, 
       {
         ProfScope ps(P, 1, ss);
         OpCocgB<double> bb{r, q, N, st};
-        TRY(launch_point<double>(P, P->g64, 0, bb, rb, ss));
+        TRY(launch_point<double>(P, P->g64, bb, rb, ss));
       }
     }
     return 0;
@@ -1112,7 +1106,7 @@ static int cocg_loop(SolveCtx& c, cx<double>* r, cx<double>* q, cx<double>* P0, 
     }
     if (!resident) {  // (a resident launch leaves no update owed)
       OpCocgFinal<double> fin{P0, P1, x, N, st};
-      TRY(launch_point<double>(P, P->g64, 0, fin, rb, s));
+      TRY(launch_point<double>(P, P->g64, fin, rb, s));
     }
     CK(cudaMemcpyAsync(P->h_state, st, sizeof(KState), cudaMemcpyDeviceToHost, s));
     CK(cudaStreamSynchronize(s));
@@ -1219,7 +1213,7 @@ extern "C" int fdfd_solve(fdfd_plan* P, const fdfd_solve_opts* o, const void* J,
   {
     OpRhs<double> op{(const cx<double>*)J, o->has_guess ? (const cx<double>*)E : nullptr, c.b, c.x,
                      P->om_re, P->om_im, o->adjoint, P->g64.mask, N, c.st};
-    TRY(launch_point<double>(P, P->g64, 0, op, c.rb, s));
+    TRY(launch_point<double>(P, P->g64, op, c.rb, s));
   }
   if (!o->has_guess) CK(cudaMemsetAsync(E, 0, vbytes128, s));
   CK(cudaMemcpyAsync(P->h_state, c.st, sizeof(KState), cudaMemcpyDeviceToHost, s));
@@ -1266,7 +1260,7 @@ extern "C" int fdfd_solve(fdfd_plan* P, const fdfd_solve_opts* o, const void* J,
 
   if (o->adjoint) {
     OpAdjPost<double> post{c.x, N};
-    TRY(launch_point<double>(P, P->g64, 0, post, c.rb, s));
+    TRY(launch_point<double>(P, P->g64, post, c.rb, s));
   }
   // final FP64 check against the unmasked right-hand side
   TRY(residual_into(P, E, J, o->adjoint, d_res, c.rb, s));
@@ -1297,7 +1291,7 @@ extern "C" int fdfd_eps_gradient(fdfd_plan* P, const void* E, const void* E_adj,
   cudaStream_t s = (cudaStream_t)stream;
   P->launches = 0;
   OpEpsGrad<double> op{(const cx<double>*)E, (const cx<double>*)E_adj, grad, P->w2, P->g64.mask, (int)P->N};
-  return launch_point<double>(P, P->g64, 0, op, RedBuf{nullptr, nullptr}, s);
+  return launch_point<double>(P, P->g64, op, RedBuf{nullptr, nullptr}, s);
 }
 
 // ------------------------------------------------------------------ E -> H, Poynting
@@ -1312,23 +1306,9 @@ extern "C" int fdfd_e2h(fdfd_plan* P, const void* E, void* H, void* S, int32_t f
   cudaStream_t s = (cudaStream_t)stream;
   P->launches = 0;
   const cx<double> inv_miw = mkc<double>(P->om_im / m2, P->om_re / m2);  // 1 / (-i omega)
-  const Tiling t = make_tiling(P, 0);
-  const Geo<double> g = geo_with(P->g64, t);
-  const long long units = (long long)t.ntz * t.nty * P->X;
-  const cx<double>* e = (const cx<double>*)E;
-  cx<double>* h = (cx<double>*)H;
-  cx<double>* sv = (cx<double>*)S;
-  if (P->flat) {
-    auto kern = k_e2h<1, FLAT_TY>;
-    static const int occ = occupancy(kern, FLAT_TY);
-    kern<<<(unsigned)std::min(units, (long long)occ * P->nsm), dim3(1, FLAT_TY), 0, s>>>(g, e, h, sv, inv_miw,
-                                                                                       conj_h, h_in);
-  } else {
-    auto kern = k_e2h<TZ3, TY3>;
-    static const int occ = occupancy(kern, TZ3 * TY3);
-    kern<<<(unsigned)std::min(units, (long long)occ * P->nsm), dim3(TZ3, TY3), 0, s>>>(g, e, h, sv, inv_miw,
-                                                                                        conj_h, h_in);
-  }
+  static const int occ = occupancy(k_e2h, POINT_NT);
+  k_e2h<<<point_blocks(P, occ), POINT_NT, 0, s>>>(P->g64, P->cells, (const cx<double>*)E, (cx<double>*)H, (cx<double>*)S,
+                                                 inv_miw, conj_h, h_in);
   P->launches++;
   CKL();
   return 0;

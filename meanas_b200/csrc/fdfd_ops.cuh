@@ -1053,20 +1053,18 @@ struct OpTfsf {
 // (conj_h, the product meanas/test/test_fdfd.py:38-40 forms) or H (H itself the
 // caller's when h_in: functional.poynting_e_cross_h(dxes)(E, H)), on the Yee grid of
 // meanas/fdfd/functional.py:187-221: E components weighted by dx_e and taken one cell
-// up along the cross axis, H components weighted by dx_h.  One thread per cell over
-// (x plane, y/z tile) units like the pointwise engine; E's +1 neighbours come through
-// L1/L2, so HBM sees E once and H, S once each.
-template <int TZ, int TY>
-__global__ void __launch_bounds__(TZ * TY) k_e2h(const Geo<double> g, const cx<double>* __restrict__ E,
-                                                 cx<double>* __restrict__ H, cx<double>* __restrict__ S,
-                                                 cx<double> inv_miw, int conj_h, int h_in) {
+// up along the cross axis, H components weighted by dx_h.  Cells to threads by number as in
+// the pointwise engine; E's +1 neighbours come through L1/L2, so HBM sees E once and H, S once
+// each: 160x160x128 84.8 us (5.6 TB/s; 88 with tiles), 121x97x109 with mu and PMC 50 (53.5).
+__global__ void __launch_bounds__(POINT_NT) k_e2h(const Geo<double> g, const CellDiv cd,
+                                                  const cx<double>* __restrict__ E, cx<double>* __restrict__ H,
+                                                  cx<double>* __restrict__ S, cx<double> inv_miw, int conj_h,
+                                                  int h_in) {
   using C = cx<double>;
-  const int ntiles = g.ntz * g.nty, units = ntiles * g.X, YZ = g.Y * g.Z, N = g.N;
-  for (int u = blockIdx.x; u < units; u += gridDim.x) {
-    const int i = u / ntiles, t = u - i * ntiles;
-    const int tyb = t / g.ntz, tzb = t - tyb * g.ntz;
-    const int j = tyb * TY + threadIdx.y, k = tzb * TZ + threadIdx.x;
-    if (j >= g.Y || k >= g.Z) continue;
+  const int YZ = g.Y * g.Z, N = g.N;
+  for (long long n = (long long)blockIdx.x * POINT_NT + threadIdx.x; n < N; n += (long long)gridDim.x * POINT_NT) {
+    int i, j, k;
+    cd((int)n, i, j, k);
     const int i1 = i + 1 == g.X ? 0 : i + 1, j1 = j + 1 == g.Y ? 0 : j + 1, k1 = k + 1 == g.Z ? 0 : k + 1;
     const int c0 = i * YZ + j * g.Z + k;
     const int cx1 = i1 * YZ + j * g.Z + k, cy1 = i * YZ + j1 * g.Z + k, cz1 = i * YZ + j * g.Z + k1;
