@@ -383,7 +383,6 @@ static int launch_point(fdfd_plan* P, const Geo<R>& g, const Op& op, RedBuf rb, 
 }
 
 // ------------------------------------------------------------------ resident solves
-static constexpr int RES_NT = 512;     // 128 registers a thread (576 to 768 threads spill more and are slower)
 static constexpr int RES_CHUNK = 256;  // iterations per launch: a millisecond or two between polls
 
 // The brick split with the least work on the largest brick among those of at most one CTA
@@ -391,7 +390,7 @@ static constexpr int RES_CHUNK = 256;  // iterations per launch: a millisecond o
 // thread.  Work: an own cell takes part in every pass, a shell cell and an H cell in one or
 // two.
 template <typename R>
-static ResidentPlan plan_resident(const fdfd_plan* P, int nshell, size_t smem_max) {
+static ResidentPlan plan_resident(const fdfd_plan* P, int nshell, int nred, size_t smem_max) {
   ResidentPlan best{};
   long long best_cost = -1;
   const int most = std::min(P->nsm, RES_CTAS);
@@ -406,7 +405,7 @@ static ResidentPlan plan_resident(const fdfd_plan* P, int nshell, size_t smem_ma
         const int kz = P->flat ? 0 : 1;
         const long long box = (long long)(bx + 2) * (by + 2) * (bz + 2 * kz);
         const long long hbox = (long long)(bx + 1) * (by + 1) * (bz + kz);
-        const size_t smem = resident_layout<R>(nshell, P->flat, bx, by, bz).total;
+        const size_t smem = resident_layout<R>(nshell, nred, P->flat, bx, by, bz).total;
         if (smem > smem_max) continue;
         const long long cost = own + box + hbox;
         if (best_cost < 0 || cost < best_cost) {
@@ -436,27 +435,28 @@ static int launch_resident(fdfd_plan* P, void (*kern)(KArgs...), const ResidentP
   return 0;
 }
 
-template <bool FLAT>
+// The instance of a resident kernel for a plan: cells per thread, flat, materials.
+#define RES_PICK(name, k, flat, mat)                                                                              \
+  ((k) == 1 ? ((flat) ? ((mat) ? name<RES_NT, 1, true, true> : name<RES_NT, 1, true, false>)                      \
+                      : ((mat) ? name<RES_NT, 1, false, true> : name<RES_NT, 1, false, false>))                   \
+            : ((flat) ? ((mat) ? name<RES_NT, 2, true, true> : name<RES_NT, 2, true, false>)                      \
+                      : ((mat) ? name<RES_NT, 2, false, true> : name<RES_NT, 2, false, false>)))
+
 static int launch_cocg_resident(fdfd_plan* P, cx<double>* r, cx<double>* p, cx<double>* x, Word* surface, KState* st,
                                 ResidentScratch* gs, unsigned long long tag, int nit, cudaStream_t s) {
   const ResidentPlan& rp = P->res_cocg;
   CK(cudaMemsetAsync(gs->counter, 0, sizeof(gs->counter), s));
-  if (rp.k == 1)
-    return launch_resident(P, k_cocg_resident<RES_NT, 1, FLAT>, rp, s, P->g64, rp.bk, r, p, x, surface, st, gs, tag, nit);
-  return launch_resident(P, k_cocg_resident<RES_NT, 2, FLAT>, rp, s, P->g64, rp.bk, r, p, x, surface, st, gs, tag, nit);
+  return launch_resident(P, RES_PICK(k_cocg_resident, rp.k, P->flat, P->has_mu || P->has_mask), rp, s, P->g64, rp.bk, r,
+                         p, x, surface, st, gs, tag, nit);
 }
 
-template <bool FLAT>
 static int launch_bicgstab_resident(fdfd_plan* P, cx<float>* r, cx<float>* p, cx<float>* x, Word* surface,
                                     unsigned seed, KState* st, ResidentScratch* gs, unsigned long long tag, int nit,
                                     cudaStream_t s) {
   const ResidentPlan& rp = P->res_bs;
   CK(cudaMemsetAsync(gs->counter, 0, sizeof(gs->counter), s));
-  if (rp.k == 1)
-    return launch_resident(P, k_bicgstab_resident<RES_NT, 1, FLAT>, rp, s, P->g32, rp.bk, r, p, x, surface, seed, st,
-                           gs, tag, nit);
-  return launch_resident(P, k_bicgstab_resident<RES_NT, 2, FLAT>, rp, s, P->g32, rp.bk, r, p, x, surface, seed, st, gs,
-                         tag, nit);
+  return launch_resident(P, RES_PICK(k_bicgstab_resident, rp.k, P->flat, P->has_mu || P->has_mask), rp, s, P->g32, rp.bk,
+                         r, p, x, surface, seed, st, gs, tag, nit);
 }
 
 #define TRY(x)                 \
@@ -631,8 +631,8 @@ extern "C" int fdfd_plan_create(const fdfd_grid_desc* d, void* ws, size_t ws_byt
     cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev);
     P->smem_optin = (size_t)optin;
     if (coop) {
-      P->res_cocg = plan_resident<double>(P, 1, P->smem_optin);
-      if (P->has32) P->res_bs = plan_resident<float>(P, 4, P->smem_optin);
+      P->res_cocg = plan_resident<double>(P, 1, COCG_SUMS, P->smem_optin);
+      if (P->has32) P->res_bs = plan_resident<float>(P, 4, BS_SUMS, P->smem_optin);
     }
   }
   auto cleanup = [&](int rc) {
@@ -1004,10 +1004,7 @@ static int refine_loop(SolveCtx& c, const Geo<RI>& gi, int prec, BsBufs B, doubl
         TRY(drive(P, sti, nit, hi.maxiter, s, [&]() -> int {
           const unsigned long long tag = c.tag;
           c.tag += (unsigned long long)nit;
-          return P->flat ? launch_bicgstab_resident<true>(P, (cx<RI>*)B.R0, (cx<RI>*)B.T, D, surface, seed, sti,
-                                                          c.scratch, tag, nit, s)
-                         : launch_bicgstab_resident<false>(P, (cx<RI>*)B.R0, (cx<RI>*)B.T, D, surface, seed, sti,
-                                                           c.scratch, tag, nit, s);
+          return launch_bicgstab_resident(P, (cx<RI>*)B.R0, (cx<RI>*)B.T, D, surface, seed, sti, c.scratch, tag, nit, s);
         }));
       }
     }
@@ -1092,8 +1089,7 @@ static int cocg_loop(SolveCtx& c, cx<double>* r, cx<double>* q, cx<double>* P0, 
       TRY(drive(P, st, nit, left, s, [&]() -> int {
         const unsigned long long tag = c.tag;
         c.tag += (unsigned long long)nit;
-        return P->flat ? launch_cocg_resident<true>(P, r, P0, x, c.surface, st, c.scratch, tag, nit, s)
-                       : launch_cocg_resident<false>(P, r, P0, x, c.surface, st, c.scratch, tag, nit, s);
+        return launch_cocg_resident(P, r, P0, x, c.surface, st, c.scratch, tag, nit, s);
       }));
     } else if (P->h_state->status == ST_RUNNING && left > 0) {
       TRY(drive(P, st, chunk, left, s, [&]() -> int {

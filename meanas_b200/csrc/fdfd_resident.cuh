@@ -77,24 +77,34 @@ struct ResidentScratch {
 // first half stores and arrives; the second waits for exchange `tag`, the `round`-th of
 // this launch (from 1), and leaves the totals in `out` (shared memory).  Warp r looks after
 // value r throughout.  Every thread must call both.
+//
+// Block sum: two shuffle rounds, then the quarter lanes' sums through shared memory
+// (`red`, NRED rows of RED_ROW), where warp r adds up row r.  Shuffling all the way is 10
+// shuffles per value and warp, and the SM has one shuffle unit for them.
+template <int NT>
+struct RedRow {
+  static constexpr int value = NT / 4;
+};
 template <int NT, int FIRST, int NRED>
 __device__ __forceinline__ void sums_begin(double (&v)[NRED], double* red, ResidentScratch* gs,
                                            unsigned long long tag) {
-  constexpr int NW = NT / 32;
-  static_assert(NW <= 32 && NRED <= NW && FIRST + NRED <= RES_SUMS, "");
+  constexpr int ROW = RedRow<NT>::value;
+  static_assert(NRED <= NT / 32 && FIRST + NRED <= RES_SUMS && ROW % 32 == 0, "");
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
 #pragma unroll
-  for (int o = 16; o > 0; o >>= 1) {
+  for (int o = 16; o > 4; o >>= 1) {
 #pragma unroll
     for (int r = 0; r < NRED; ++r) v[r] += __shfl_down_sync(0xffffffffu, v[r], o);
   }
-  if (lane == 0) {
+  if (lane < 8) {
 #pragma unroll
-    for (int r = 0; r < NRED; ++r) red[warp * 8 + r] = v[r];
+    for (int r = 0; r < NRED; ++r) red[r * ROW + warp * 8 + lane] = v[r];
   }
   __syncthreads();
   if (warp < NRED) {
-    double s = lane < NW ? red[lane * 8 + warp] : 0.0;
+    double s = 0.0;
+#pragma unroll
+    for (int q = 0; q < ROW; q += 32) s += red[warp * ROW + q + lane];
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) s += __shfl_down_sync(0xffffffffu, s, o);
     if (lane == 0) {
@@ -145,15 +155,24 @@ __device__ __forceinline__ bool sums_end(double* out, int* gave_up, ResidentScra
   return *gave_up == 0;
 }
 
-// a / b with one division: b scaled by a power of two so that |b|^2 neither overflows nor
-// underflows (Smith's form costs three divisions, a quarter of an iteration's scalar work).
+// 1 / d for d in [1, 8): the hardware's approximate reciprocal (better than 2^-20) and two
+// Newton steps, whose errors square (2^-40, then rounding): within an ulp or two.  A full
+// division is some 400 cycles of latency, an iteration's scalar work had six of them.
+__device__ __forceinline__ double newton_reciprocal(double d) {
+  double y;
+  asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(d));
+  y = fma(y, fma(-d, y, 1.0), y);
+  return fma(y, fma(-d, y, 1.0), y);
+}
+
+// a / b: b scaled by a power of two so that |b|^2 is in [1, 8).
 __device__ __forceinline__ dcx cdiv(dcx a, dcx b) {
   const double big = fmax(fabs(b.re), fabs(b.im));
   const int e = (__double2hiint(big) >> 20) & 0x7ff;
   if (e < 24 || e > 2022) return ddiv(a, b);
   const double sc = __hiloint2double((2046 - e) << 20, 0);  // 2^(1023 - e): big * sc in [1, 2)
   const double re = b.re * sc, im = b.im * sc;
-  const double inv = sc / fma(re, re, im * im);
+  const double inv = sc * newton_reciprocal(fma(re, re, im * im));
   return {fma(a.re, re, a.im * im) * inv, fma(a.im, re, -(a.re * im)) * inv};
 }
 
@@ -298,7 +317,7 @@ struct BrickTables {
 // H = pm mu^-1 ce(U) on the H region of a brick, U and Hs in shared memory (component
 // stride box / hbox).  An item is two cells adjacent in x, which share a third of their
 // loads: the pass is bound by shared-memory bandwidth.
-template <typename R, int NT, bool FLAT>
+template <typename R, int NT, bool FLAT, bool MAT>
 __device__ __forceinline__ void brick_curl_e(const Geo<R>& g, const Brick<R, FLAT>& B, const BrickTables<R>& T,
                                              const cx<R>* U, cx<R>* Hs) {
   const cx<R>* Ux = U;
@@ -331,7 +350,7 @@ __device__ __forceinline__ void brick_curl_e(const Geo<R>& g, const Brick<R, FLA
         hy = dzux - dxuz;
         hz = dxuy - dyux;
       }
-      if (g.muinv || g.mask) {
+      if (MAT) {
         int ci = B.i0 + i - 1, cj = B.j0 + j - 1, ck = B.k0 + k - Brick<R, FLAT>::KZ;
         ci = ci < 0 ? g.X - 1 : ci;
         cj = cj < 0 ? g.Y - 1 : cj;
@@ -387,7 +406,7 @@ __device__ __forceinline__ OwnCells<K> own_cells(const Geo<R>& g, const Brick<R,
 }
 
 // y = A0 u on a thread's own cells; cells on the brick's surface also go to their words.
-template <typename R, int K, bool FLAT>
+template <typename R, int K, bool FLAT, bool MAT>
 __device__ __forceinline__ void brick_curl_h(const Geo<R>& g, const Brick<R, FLAT>& B, const BrickTables<R>& T,
                                              const cx<R>* U, const cx<R>* Hs, cx<R> w2, const OwnCells<K>& o,
                                              cx<R> (&y)[K][3], Word* surface, unsigned long long tag) {
@@ -412,7 +431,7 @@ __device__ __forceinline__ void brick_curl_h(const Geo<R>& g, const Brick<R, FLA
       y[m][1] = (hx - Hx[h - 1]) * idzh - (hz - hz_prev) * idxh;
     }
     y[m][2] = (hy - hy_prev) * idxh - (hx - Hx[h - B.hz]) * idyh;
-    const uint8_t mk = g.mask ? __ldg(g.mask + cell) : (uint8_t)0;
+    const uint8_t mk = MAT && g.mask ? __ldg(g.mask + cell) : (uint8_t)0;
 #pragma unroll
     for (int c = 0; c < 3; ++c) {
       const cx<R> v = y[m][c] - (__ldg(g.eps + c * g.N + cell) * w2) * U[c * B.box + o.pos + m * B.sy];
@@ -456,12 +475,14 @@ __device__ __forceinline__ void list_shell(const Geo<R>& g, const Brick<R, FLAT>
 }
 
 // Shared memory of a resident solve: the box vector U, `nshell` vectors on the shell, the H
-// region, the shell list, the tables and the exchange scratch.
+// region, the shell list, the tables and the exchange scratch (of at
+// most `nred` sums at once).
 struct ResidentLayout {
   size_t shell_vec, h, shell, tables, red, total;
 };
+constexpr int RES_NT = 512;  // threads: 128 registers each (576 to 768 threads spill more and are slower)
 template <typename R>
-__host__ __device__ inline ResidentLayout resident_layout(int nshell, bool flat, int bx, int by, int bz) {
+__host__ __device__ inline ResidentLayout resident_layout(int nshell, int nred, bool flat, int bx, int by, int bz) {
   const size_t kz = flat ? 0 : 1;
   const size_t box = (size_t)(bx + 2) * (by + 2) * (bz + 2 * kz), own = (size_t)bx * by * bz;
   const size_t hbox = (size_t)(bx + 1) * (by + 1) * (bz + kz);
@@ -471,7 +492,7 @@ __host__ __device__ inline ResidentLayout resident_layout(int nshell, bool flat,
   L.shell = (L.h + sizeof(cx<R>) * 3 * hbox + 15) & ~(size_t)15;
   L.tables = L.shell + ((sizeof(int2) * (box - own) + 15) & ~(size_t)15);
   L.red = L.tables + ((BrickTables<R>::bytes(bx, by, bz) + 15) & ~(size_t)15);
-  L.total = L.red + (32 * 8 + 2 * RES_SUMS + 2) * sizeof(double);
+  L.total = L.red + ((size_t)nred * RedRow<RES_NT>::value + 2 * RES_SUMS + 2) * sizeof(double);
   return L;
 }
 
@@ -486,12 +507,13 @@ __host__ __device__ inline ResidentLayout resident_layout(int nshell, bool flat,
 // thread in registers.  `surface`: two buffers (even and odd tags) of 6 N words, since the
 // shell is read while the second exchange is under way.
 //
-// Measured per iteration, two launches / resident: 16^3 25.0 / 6.3 us, 32^3 25.6 / 7.6,
-// 48^3 30.3 / 13.9, 52^3 (the largest cube that fits) 37.4 / 17.6; flat 128^2 23.4 / 6.5,
-// 380^2 34.2 / 11.8.  It is bound by the exchanges (about 3.3 us of each iteration) and, on
-// full bricks, by shared-memory bandwidth in the two curl passes.  512 threads: 576 to 768
-// leave 80 to 96 registers and spill (48^3: 15.3 us).
-template <int NT, int K, bool FLAT>
+// Measured per iteration, two launches / resident: 16^3 25.0 / 5.9 us, 40^3 28.5 / 9.9, 52^3
+// (the largest cube that fits) 37.4 / 16.9; flat 128^2 23.4 / 6.1, 380^2 34.2 / 11.0.  It is
+// bound by the exchanges (about 3 us of each iteration) and, on full bricks, by shared-memory
+// bandwidth in the two curl passes.  Of that, dividing by newton_reciprocal, block sums through
+// shared memory and material code by template gave 0.4 to 0.8 us.
+constexpr int COCG_SUMS = 5;
+template <int NT, int K, bool FLAT, bool MAT>
 __global__ void __launch_bounds__(NT, 1)
     k_cocg_resident(const Geo<double> g, const Bricks bk, cx<double>* r, cx<double>* p, cx<double>* x, Word* surface,
                     KState* st, ResidentScratch* gs, unsigned long long tag0, int nit) {
@@ -499,7 +521,7 @@ __global__ void __launch_bounds__(NT, 1)
   using C = cx<R>;
   if (ld_status(st) != ST_RUNNING) return;
   extern __shared__ __align__(16) unsigned char smem_raw[];
-  const ResidentLayout L = resident_layout<R>(1, FLAT, bk.bx, bk.by, bk.bz);
+  const ResidentLayout L = resident_layout<R>(1, COCG_SUMS, FLAT, bk.bx, bk.by, bk.bz);
   Brick<R, FLAT> B;
   B.init(g, bk);
   C* P = reinterpret_cast<C*>(smem_raw);
@@ -509,7 +531,7 @@ __global__ void __launch_bounds__(NT, 1)
   BrickTables<R> T;
   T.carve(smem_raw + L.tables, bk.bx, bk.by, bk.bz);
   double* red = reinterpret_cast<double*>(smem_raw + L.red);
-  double* sums = red + 32 * 8;
+  double* sums = red + COCG_SUMS * RedRow<NT>::value;
   int* flags = reinterpret_cast<int*>(sums + 2 * RES_SUMS);  // [0] shell count, [1] gave up
   const int tid = threadIdx.x, N = g.N, YZ = g.Y * g.Z;
   if (tid == 0) flags[0] = flags[1] = 0;
@@ -557,7 +579,7 @@ __global__ void __launch_bounds__(NT, 1)
   // shell entries go round from the first thread without own cells
   const int rows = B.ly * B.lz, items = ((B.lx + K - 1) / K) * rows;
   const int spare = tid >= items ? tid - items : tid - items + NT;
-  constexpr int NRHO = 5;
+  constexpr int NRHO = COCG_SUMS;
   for (int it = 0; it < nit; ++it) {
     const unsigned long long tag = tag0 + (unsigned long long)it + 1;
     Word* const sw = surface + (tag & 1) * SurfaceRows<R>::value * (size_t)N;
@@ -579,9 +601,9 @@ __global__ void __launch_bounds__(NT, 1)
     }
     owed = false;
     __syncthreads();
-    brick_curl_e<R, NT, FLAT>(g, B, T, P, Hs);
+    brick_curl_e<R, NT, FLAT, MAT>(g, B, T, P, Hs);
     __syncthreads();
-    brick_curl_h<R, K, FLAT>(g, B, T, P, Hs, w2, o, t, sw, tag);
+    brick_curl_h<R, K, FLAT, MAT>(g, B, T, P, Hs, w2, o, t, sw, tag);
     {
       double acc[2] = {0.0, 0.0};
       WeightYZ<R> wyz;
@@ -716,10 +738,11 @@ __global__ void __launch_bounds__(NT, 1)
 // shells are read before the sums that their writers wait for, so each product has one
 // buffer of 3 N words.
 //
-// Measured per iteration, two launches / resident: 16^3 29.6 / 7.6 us, 40^3 33.6 / 10.2,
-// 52^3 (the largest cube that fits) 44.2 / 15.1; flat 128^2 29.7 / 7.4, 380^2 39.6 / 10.7.
+// Measured per iteration, two launches / resident: 16^3 29.6 / 6.8 us, 40^3 33.6 / 9.5, 52^3
+// (the largest cube that fits) 44.2 / 14.0; flat 128^2 29.7 / 6.7, 380^2 39.6 / 9.9.
 // Bound as COCG is: two exchanges, then shared-memory bandwidth on full bricks.
-template <int NT, int K, bool FLAT>
+constexpr int BS_SUMS = 6;
+template <int NT, int K, bool FLAT, bool MAT>
 __global__ void __launch_bounds__(NT, 1)
     k_bicgstab_resident(const Geo<float> g, const Bricks bk, cx<float>* r, cx<float>* p, cx<float>* x, Word* surface,
                         unsigned seed, KState* st, ResidentScratch* gs, unsigned long long tag0, int nit) {
@@ -727,7 +750,7 @@ __global__ void __launch_bounds__(NT, 1)
   using C = cx<R>;
   if (ld_status(st) != ST_RUNNING) return;
   extern __shared__ __align__(16) unsigned char smem_raw[];
-  const ResidentLayout L = resident_layout<R>(4, FLAT, bk.bx, bk.by, bk.bz);
+  const ResidentLayout L = resident_layout<R>(4, BS_SUMS, FLAT, bk.bx, bk.by, bk.bz);
   Brick<R, FLAT> B;
   B.init(g, bk);
   C* U = reinterpret_cast<C*>(smem_raw);
@@ -741,7 +764,7 @@ __global__ void __launch_bounds__(NT, 1)
   BrickTables<R> T;
   T.carve(smem_raw + L.tables, bk.bx, bk.by, bk.bz);
   double* red = reinterpret_cast<double*>(smem_raw + L.red);
-  double* sums = red + 32 * 8;
+  double* sums = red + BS_SUMS * RedRow<NT>::value;
   int* flags = reinterpret_cast<int*>(sums + 2 * RES_SUMS);
   const int tid = threadIdx.x, N = g.N, YZ = g.Y * g.Z;
   if (tid == 0) flags[0] = flags[1] = 0;
@@ -786,7 +809,7 @@ __global__ void __launch_bounds__(NT, 1)
   // shell entries go round from the first thread without own cells
   const int items = ((B.lx + K - 1) / K) * B.ly * B.lz;
   const int spare = tid >= items ? tid - items : tid - items + NT;
-  constexpr int NS = 2, NT6 = 6;
+  constexpr int NS = 2, NT6 = BS_SUMS;
   for (int it = 0; it < nit; ++it) {
     const unsigned long long tag = tag0 + (unsigned long long)it + 1;
     C alpha, omega, beta;
@@ -802,9 +825,9 @@ __global__ void __launch_bounds__(NT, 1)
       for (int c = 0; c < 3; ++c) U[c * B.box + pos] = Ps[c * nshell + e];
     }
     __syncthreads();
-    brick_curl_e<R, NT, FLAT>(g, B, T, U, Hs);
+    brick_curl_e<R, NT, FLAT, MAT>(g, B, T, U, Hs);
     __syncthreads();
-    brick_curl_h<R, K, FLAT>(g, B, T, U, Hs, w2, o, vv, surface, tag);
+    brick_curl_h<R, K, FLAT, MAT>(g, B, T, U, Hs, w2, o, vv, surface, tag);
     {
       R a[2] = {R(0), R(0)};
 #pragma unroll
@@ -852,9 +875,9 @@ __global__ void __launch_bounds__(NT, 1)
       }
     }
     __syncthreads();
-    brick_curl_e<R, NT, FLAT>(g, B, T, U, Hs);
+    brick_curl_e<R, NT, FLAT, MAT>(g, B, T, U, Hs);
     __syncthreads();
-    brick_curl_h<R, K, FLAT>(g, B, T, U, Hs, w2, o, tv, surface + SurfaceRows<R>::value * nw, tag);
+    brick_curl_h<R, K, FLAT, MAT>(g, B, T, U, Hs, w2, o, tv, surface + SurfaceRows<R>::value * nw, tag);
     {
       R a[NT6] = {R(0), R(0), R(0), R(0), R(0), R(0)};
 #pragma unroll
