@@ -620,18 +620,23 @@ __device__ __forceinline__ void stencil_unit(const Geo<R>& g, const Op& o, RedBu
     const cx<R>* Uy = U + (cur * 3 + 1) * BOX;
     const cx<R>* Uz = U + (cur * 3 + 2) * BOX;
     const int p = bj * BW + bk;
+    // (all loads before the arithmetic: left to the compiler's order, COCG's pass took 191
+    // instead of 188 us at 160x160x128, 145 instead of 140 at 121x97x109 with masks)
     const cx<R> ux = Ux[p], uy = Uy[p], uz = Uz[p];
-    const cx<R> dyuz = (Uz[p + BW] - uz) * idy;
-    const cx<R> dyux = (Ux[p + BW] - ux) * idy;
-    const cx<R> dxuz = (U[(nxt * 3 + 2) * BOX + p] - uz) * idx_e;
-    const cx<R> dxuy = (U[(nxt * 3 + 1) * BOX + p] - uy) * idx_e;
+    const cx<R> uz_i = U[(nxt * 3 + 2) * BOX + p], uy_i = U[(nxt * 3 + 1) * BOX + p];
+    const cx<R> uz_j = Uz[p + BW], ux_j = Ux[p + BW];
+    const cx<R> uy_k = FLAT ? czero<R>() : Uy[p + 1], ux_k = FLAT ? czero<R>() : Ux[p + 1];
+    const cx<R> dyuz = (uz_j - uz) * idy;
+    const cx<R> dyux = (ux_j - ux) * idy;
+    const cx<R> dxuz = (uz_i - uz) * idx_e;
+    const cx<R> dxuy = (uy_i - uy) * idx_e;
     if (FLAT) {
       hx = dyuz;
       hy = czero<R>() - dxuz;
       hz = dxuy - dyux;
     } else {
-      const cx<R> dzuy = (Uy[p + 1] - uy) * idz;
-      const cx<R> dzux = (Ux[p + 1] - ux) * idz;
+      const cx<R> dzuy = (uy_k - uy) * idz;
+      const cx<R> dzux = (ux_k - ux) * idz;
       hx = dyuz - dzuy;
       hy = dzux - dxuz;
       hz = dxuy - dyux;
