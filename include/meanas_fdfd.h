@@ -96,7 +96,8 @@ typedef struct fdfd_solve_opts {
   double* history;       /* optional device float64[maxiter + 1]: relative residuals */
   int32_t profile;       /* nonzero: time every iteration kernel with CUDA events (no
                             graphs); fills the *_ms / *_launches fields of the info  */
-  int32_t pad_;
+  int32_t wait_limit;    /* reads of a word after which a CTA of a resident solve stops waiting for
+                            the others (0 = default, one to two seconds)            */
 } fdfd_solve_opts;
 
 typedef struct fdfd_solve_info {

@@ -57,7 +57,7 @@ class SolveOpts(C.Structure):
         ('inner_rtol', C.c_double),
         ('history', C.c_void_p),
         ('profile', C.c_int32),
-        ('pad_', C.c_int32),
+        ('wait_limit', C.c_int32),
     ]
 
 

@@ -443,20 +443,20 @@ static int launch_resident(fdfd_plan* P, void (*kern)(KArgs...), const ResidentP
                       : ((mat) ? name<RES_NT, 2, false, true> : name<RES_NT, 2, false, false>)))
 
 static int launch_cocg_resident(fdfd_plan* P, cx<double>* r, cx<double>* p, cx<double>* x, Word* surface, KState* st,
-                                ResidentScratch* gs, unsigned long long tag, int nit, cudaStream_t s) {
+                                ResidentScratch* gs, unsigned long long tag, int nit, int limit, cudaStream_t s) {
   const ResidentPlan& rp = P->res_cocg;
   CK(cudaMemsetAsync(gs->counter, 0, sizeof(gs->counter), s));
   return launch_resident(P, RES_PICK(k_cocg_resident, rp.k, P->flat, P->has_mu || P->has_mask), rp, s, P->g64, rp.bk, r,
-                         p, x, surface, st, gs, tag, nit);
+                         p, x, surface, st, gs, tag, nit, limit);
 }
 
 static int launch_bicgstab_resident(fdfd_plan* P, cx<float>* r, cx<float>* p, cx<float>* x, Word* surface,
                                     unsigned seed, KState* st, ResidentScratch* gs, unsigned long long tag, int nit,
-                                    cudaStream_t s) {
+                                    int limit, cudaStream_t s) {
   const ResidentPlan& rp = P->res_bs;
   CK(cudaMemsetAsync(gs->counter, 0, sizeof(gs->counter), s));
   return launch_resident(P, RES_PICK(k_bicgstab_resident, rp.k, P->flat, P->has_mu || P->has_mask), rp, s, P->g32, rp.bk,
-                         r, p, x, surface, seed, st, gs, tag, nit);
+                         r, p, x, surface, seed, st, gs, tag, nit, limit);
 }
 
 #define TRY(x)                 \
@@ -913,6 +913,7 @@ struct SolveCtx {
   ResidentScratch* scratch;  // of resident solves, and the number of their last exchange
   unsigned long long tag;
   Word* surface;   // their surface words (two buffers of all cells), null: no room for them
+  int limit;       // reads of a word before a CTA of theirs gives up
   cx<double>* b;
   cx<double>* x;   // the caller's E
   cx<double>* e2;  // partner of E for the refinement ping-pong
@@ -1004,7 +1005,7 @@ static int refine_loop(SolveCtx& c, const Geo<RI>& gi, int prec, BsBufs B, doubl
         TRY(drive(P, sti, nit, hi.maxiter, s, [&]() -> int {
           const unsigned long long tag = c.tag;
           c.tag += (unsigned long long)nit;
-          return launch_bicgstab_resident(P, (cx<RI>*)B.R0, (cx<RI>*)B.T, D, surface, seed, sti, c.scratch, tag, nit, s);
+          return launch_bicgstab_resident(P, (cx<RI>*)B.R0, (cx<RI>*)B.T, D, surface, seed, sti, c.scratch, tag, nit, c.limit, s);
         }));
       }
     }
@@ -1023,7 +1024,7 @@ static int refine_loop(SolveCtx& c, const Geo<RI>& gi, int prec, BsBufs B, doubl
     CK(cudaMemcpyAsync(P->h_state, sti, sizeof(KState), cudaMemcpyDeviceToHost, s));
     CK(cudaStreamSynchronize(s));
     c.iters += P->h_state->iter;
-    if (P->h_state->status == ST_TIMEOUT) return set_err(FDFD_ERR_CUDA, "a CTA of a resident solve did not arrive in time");
+    if (P->h_state->timed_out) return set_err(FDFD_ERR_CUDA, "a CTA of a resident solve did not arrive in time");
     if (P->h_state->status == ST_NONFINITE) { c.status = ST_NONFINITE; break; }
     have_d = true;
   }
@@ -1089,7 +1090,7 @@ static int cocg_loop(SolveCtx& c, cx<double>* r, cx<double>* q, cx<double>* P0, 
       TRY(drive(P, st, nit, left, s, [&]() -> int {
         const unsigned long long tag = c.tag;
         c.tag += (unsigned long long)nit;
-        return launch_cocg_resident(P, r, P0, x, c.surface, st, c.scratch, tag, nit, s);
+        return launch_cocg_resident(P, r, P0, x, c.surface, st, c.scratch, tag, nit, c.limit, s);
       }));
     } else if (P->h_state->status == ST_RUNNING && left > 0) {
       TRY(drive(P, st, chunk, left, s, [&]() -> int {
@@ -1108,7 +1109,7 @@ static int cocg_loop(SolveCtx& c, cx<double>* r, cx<double>* q, cx<double>* P0, 
     CK(cudaStreamSynchronize(s));
     c.iters += P->h_state->iter;
     c.status = P->h_state->status;
-    if (c.status == ST_TIMEOUT) return set_err(FDFD_ERR_CUDA, "a CTA of a resident solve did not arrive in time");
+    if (P->h_state->timed_out) return set_err(FDFD_ERR_CUDA, "a CTA of a resident solve did not arrive in time");
     if (c.status == ST_RUNNING) c.status = ST_MAXITER;
     if (c.status != ST_BREAKDOWN || restarts >= 8 || c.iters >= maxiter) break;
     // Breakdown: the unconjugated form cancelled (for example a source whose
@@ -1180,6 +1181,7 @@ extern "C" int fdfd_solve(fdfd_plan* P, const fdfd_solve_opts* o, const void* J,
   c.scratch = (ResidentScratch*)(base + L.scratch);
   c.tag = 0;
   c.surface = nullptr;
+  c.limit = o->wait_limit > 0 ? o->wait_limit : SPIN_LIMIT;
   c.b = (cx<double>*)(base + L.b);
   c.x = (cx<double>*)E;
   c.e2 = (cx<double>*)(base + L.e2);

@@ -57,7 +57,7 @@ struct KState {
                    // best residual (0 = never)
   double best_rr;  // BiCGSTAB: best recurrence residual so far, and its iteration
   int best_iter;
-  int pad2;
+  int timed_out;   // set by any CTA of a resident launch whose wait ran out
   double* hist;    // relative residual history (length maxiter + 1) or null
 };
 

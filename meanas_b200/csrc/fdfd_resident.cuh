@@ -25,15 +25,19 @@
 //
 // Reuse of words: a CTA writes its words of the next exchange of a kind only after the
 // other exchange in between has completed, which all readers entered after reading.
-// Every wait is bounded: after SPIN_LIMIT reads a CTA gives up, reports ST_TIMEOUT and
-// returns (the launch is cooperative, so its CTAs do run at the same time).
+// Every wait is bounded: after `limit` reads (SPIN_LIMIT, or the caller's; SPIN_LIMIT in the
+// first exchange of a launch, which waits for the launch itself) a CTA gives up, sets
+// KState::timed_out and returns (the launch is cooperative, so its CTAs do run at the same
+// time).  The others may have got past that exchange, converged even, so the flag and not the
+// status that CTA 0 writes says whether the vectors belong together; launches that find it set
+// do nothing.
 #pragma once
 #include "fdfd_ops.cuh"
 
 namespace fdfd {
 
 constexpr int ST_TIMEOUT = 5;
-constexpr int SPIN_LIMIT = 1 << 22;
+constexpr int SPIN_LIMIT = 1 << 22;  // one to two seconds
 
 // Bricks of the grid: nx x ny x nz of them, at most bx x by x bz cells each (the split of
 // an axis is balanced: brick i covers [i n / m, (i + 1) n / m)).
@@ -116,7 +120,7 @@ __device__ __forceinline__ void sums_begin(double (&v)[NRED], double* red, Resid
 
 template <int FIRST, int NRED>
 __device__ __forceinline__ bool sums_end(double* out, int* gave_up, ResidentScratch* gs, unsigned long long tag,
-                                         unsigned int round) {
+                                         unsigned int round, int limit) {
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   if (warp < NRED) {
     bool ok = true;
@@ -126,7 +130,7 @@ __device__ __forceinline__ bool sums_end(double* out, int* gave_up, ResidentScra
       int spin = 0;
       do {
         asm volatile("ld.relaxed.gpu.global.u32 %0, [%1];" : "=r"(n) : "l"(&gs->counter[FIRST + warp][0]) : "memory");
-      } while (n < all && ++spin < SPIN_LIMIT);
+      } while (n < all && ++spin < limit);
       ok = n >= all;
     }
     __syncwarp();
@@ -135,13 +139,14 @@ __device__ __forceinline__ bool sums_end(double* out, int* gave_up, ResidentScra
     const int last = (int)gridDim.x - 1;
     Word got[M];
     bool here = false;
-    for (int spin = 0; spin < SPIN_LIMIT && !here; ++spin) {
+    int spin = 0;
+    do {
 #pragma unroll
       for (int m = 0; m < M; ++m) got[m] = word_load(w + min(lane + 32 * m, last));
       here = true;
 #pragma unroll
       for (int m = 0; m < M; ++m) here = here && got[m].tag == tag;
-    }
+    } while (!here && ++spin < limit);
     double s = 0.0;
 #pragma unroll
     for (int m = 0; m < M; ++m)
@@ -196,17 +201,19 @@ __device__ __forceinline__ void surface_store(Word* w, size_t n, int cell, const
   for (int c = 0; c < 3; ++c) word_store(w + c * n + cell, pack(v[c].re, v[c].im), tag);
 }
 template <typename R>
-__device__ __forceinline__ bool surface_load(const Word* w, size_t n, int cell, cx<R> v[3], unsigned long long tag) {
+__device__ __forceinline__ bool surface_load(const Word* w, size_t n, int cell, cx<R> v[3], unsigned long long tag,
+                                             int limit) {
   constexpr int NR = SurfaceRows<R>::value;
   Word a[NR];
   bool ok = false;
-  for (int spin = 0; spin < SPIN_LIMIT && !ok; ++spin) {
+  int spin = 0;
+  do {
 #pragma unroll
     for (int q = 0; q < NR; ++q) a[q] = word_load(w + q * n + cell);
     ok = true;
 #pragma unroll
     for (int q = 0; q < NR; ++q) ok = ok && a[q].tag == tag;
-  }
+  } while (!ok && ++spin < limit);
 #pragma unroll
   for (int c = 0; c < 3; ++c) {
     if constexpr (sizeof(R) == 8) {
@@ -216,6 +223,18 @@ __device__ __forceinline__ bool surface_load(const Word* w, size_t n, int cell, 
     }
   }
   return ok;
+}
+
+// Whether a launch has work.  One thread looks and the CTA follows: a CTA may start while
+// others give up already.
+__device__ __forceinline__ bool resident_begin(KState* st) {
+  bool go = true;
+  if (threadIdx.x == 0) {
+    const bool lost = *(volatile const int*)&st->timed_out != 0;
+    go = ld_status(st) == ST_RUNNING && !lost;
+    if (lost && blockIdx.x == 0) st->status = ST_TIMEOUT;  // the host looks here between launches
+  }
+  return __syncthreads_and(go) != 0;
 }
 
 // ------------------------------------------------------------------ bricks
@@ -516,10 +535,10 @@ constexpr int COCG_SUMS = 5;
 template <int NT, int K, bool FLAT, bool MAT>
 __global__ void __launch_bounds__(NT, 1)
     k_cocg_resident(const Geo<double> g, const Bricks bk, cx<double>* r, cx<double>* p, cx<double>* x, Word* surface,
-                    KState* st, ResidentScratch* gs, unsigned long long tag0, int nit) {
+                    KState* st, ResidentScratch* gs, unsigned long long tag0, int nit, int limit) {
   using R = double;
   using C = cx<R>;
-  if (ld_status(st) != ST_RUNNING) return;
+  if (!resident_begin(st)) return;
   extern __shared__ __align__(16) unsigned char smem_raw[];
   const ResidentLayout L = resident_layout<R>(1, COCG_SUMS, FLAT, bk.bx, bk.by, bk.bz);
   Brick<R, FLAT> B;
@@ -623,7 +642,7 @@ __global__ void __launch_bounds__(NT, 1)
       }
       sums_begin<NT, 0, 2>(acc, red, gs, tag);
     }
-    if (!sums_end<0, 2>(sums, &flags[1], gs, tag, it + 1)) { status = ST_TIMEOUT; break; }
+    if (!sums_end<0, 2>(sums, &flags[1], gs, tag, it + 1, it > 0 ? limit : SPIN_LIMIT)) { status = ST_TIMEOUT; break; }
     const dcx sigma = {sums[0], sums[1]};
     if (!dfinite(sigma)) { status = ST_NONFINITE; break; }
     if (sigma.re == 0.0 && sigma.im == 0.0) { status = ST_BREAKDOWN; break; }
@@ -664,11 +683,11 @@ __global__ void __launch_bounds__(NT, 1)
     }
     for (int e = tid - 32 * NRHO; e >= 0 && e < nshell; e += NT - 32 * NRHO) {
       C qv[3];
-      if (!surface_load<R>(sw, (size_t)N, shell[e].y, qv, tag)) flags[1] = 1;
+      if (!surface_load<R>(sw, (size_t)N, shell[e].y, qv, tag, limit)) flags[1] = 1;
 #pragma unroll
       for (int c = 0; c < 3; ++c) Rs[c * nshell + e] = caxpy(malpha, qv[c], Rs[c * nshell + e]);
     }
-    if (!sums_end<2, NRHO>(sums + RES_SUMS, &flags[1], gs, tag, it + 1)) { status = ST_TIMEOUT; break; }
+    if (!sums_end<2, NRHO>(sums + RES_SUMS, &flags[1], gs, tag, it + 1, limit)) { status = ST_TIMEOUT; break; }
     const double* sr = sums + RES_SUMS;
     const dcx rho_new = {sr[0], sr[1]};
     const double monitored = sr[2 + crit], pc = sr[3];
@@ -710,6 +729,7 @@ __global__ void __launch_bounds__(NT, 1)
       r[idx] = rv[m][c];
     }
   }
+  if (status == ST_TIMEOUT && tid == 0) *(volatile int*)&st->timed_out = 1;
   if (scribe) {
     if (iter > iter0) {
       st->rr = sums[RES_SUMS + 2];
@@ -745,10 +765,11 @@ constexpr int BS_SUMS = 6;
 template <int NT, int K, bool FLAT, bool MAT>
 __global__ void __launch_bounds__(NT, 1)
     k_bicgstab_resident(const Geo<float> g, const Bricks bk, cx<float>* r, cx<float>* p, cx<float>* x, Word* surface,
-                        unsigned seed, KState* st, ResidentScratch* gs, unsigned long long tag0, int nit) {
+                        unsigned seed, KState* st, ResidentScratch* gs, unsigned long long tag0, int nit,
+                        int limit) {
   using R = float;
   using C = cx<R>;
-  if (ld_status(st) != ST_RUNNING) return;
+  if (!resident_begin(st)) return;
   extern __shared__ __align__(16) unsigned char smem_raw[];
   const ResidentLayout L = resident_layout<R>(4, BS_SUMS, FLAT, bk.bx, bk.by, bk.bz);
   Brick<R, FLAT> B;
@@ -841,11 +862,11 @@ __global__ void __launch_bounds__(NT, 1)
     // while the sums travel: v of the shell, in the warps that do not wait for a sum
     for (int e = tid - 32 * NS; e >= 0 && e < nshell; e += NT - 32 * NS) {
       C q[3];
-      if (!surface_load<R>(surface, nw, shell[e].y, q, tag)) flags[1] = 1;
+      if (!surface_load<R>(surface, nw, shell[e].y, q, tag, it > 0 ? limit : SPIN_LIMIT)) flags[1] = 1;
 #pragma unroll
       for (int c = 0; c < 3; ++c) Vs[c * nshell + e] = q[c];
     }
-    if (!sums_end<0, NS>(sums, &flags[1], gs, tag, it + 1)) { status = ST_TIMEOUT; break; }
+    if (!sums_end<0, NS>(sums, &flags[1], gs, tag, it + 1, it > 0 ? limit : SPIN_LIMIT)) { status = ST_TIMEOUT; break; }
     const dcx sigma = {sums[0], sums[1]};
     if (!dfinite(sigma)) { status = ST_NONFINITE; break; }
     if ((fmax(fabs(sigma.re), fabs(sigma.im)) <= 1e-300 && dabs(sigma) <= 1e-300) ||
@@ -897,11 +918,11 @@ __global__ void __launch_bounds__(NT, 1)
     }
     for (int e = tid - 32 * NT6; e >= 0 && e < nshell; e += NT - 32 * NT6) {
       C q[3];
-      if (!surface_load<R>(surface + SurfaceRows<R>::value * nw, nw, shell[e].y, q, tag)) flags[1] = 1;
+      if (!surface_load<R>(surface + SurfaceRows<R>::value * nw, nw, shell[e].y, q, tag, limit)) flags[1] = 1;
 #pragma unroll
       for (int c = 0; c < 3; ++c) Ts[c * nshell + e] = q[c];
     }
-    if (!sums_end<NS, NT6>(sums + RES_SUMS, &flags[1], gs, tag, it + 1)) { status = ST_TIMEOUT; break; }
+    if (!sums_end<NS, NT6>(sums + RES_SUMS, &flags[1], gs, tag, it + 1, limit)) { status = ST_TIMEOUT; break; }
     const double* q = sums + RES_SUMS;
     const dcx ts = {q[0], q[1]}, rht = {q[3], q[4]};
     const double tt = q[2], ss = q[5];
@@ -972,6 +993,7 @@ __global__ void __launch_bounds__(NT, 1)
       r[idx] = rv[m][c];
     }
   }
+  if (status == ST_TIMEOUT && tid == 0) *(volatile int*)&st->timed_out = 1;
   if (scribe) {
     st->rho = rho;
     st->rr = rr;

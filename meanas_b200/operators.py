@@ -282,7 +282,7 @@ class GridOperator:
                    maxiter: int | None = None, criterion: str = 'true', adjoint: bool = False,
                    chunk: int = 0, use_graph: bool = True, inner_rtol: float = 0.0, max_outer: int = 0,
                    history: torch.Tensor | None = None, has_guess: bool = False,
-                   profile: bool = False) -> _lib.SolveOpts:
+                   profile: bool = False, wait_limit: int = 0) -> _lib.SolveOpts:
         o = _lib.SolveOpts()
         o.method = _METHODS[method]
         o.criterion = _CRITS[criterion]
@@ -298,6 +298,7 @@ class GridOperator:
         o.inner_rtol = float(inner_rtol)
         o.history = history.data_ptr() if history is not None else None
         o.profile = int(bool(profile))
+        o.wait_limit = int(wait_limit)
         return o
 
     def workspace(self, opts: _lib.SolveOpts) -> torch.Tensor:
