@@ -97,7 +97,8 @@ typedef struct fdfd_solve_opts {
   int32_t profile;       /* nonzero: time every iteration kernel with CUDA events (no
                             graphs); fills the *_ms / *_launches fields of the info  */
   int32_t wait_limit;    /* reads of a word after which a CTA of a resident solve stops waiting for
-                            the others (0 = default, one to two seconds)            */
+                            the others and the solve goes on with a launch per pass (0 =
+                            default, one to two seconds); -n: after n - 1 resident launches */
 } fdfd_solve_opts;
 
 typedef struct fdfd_solve_info {

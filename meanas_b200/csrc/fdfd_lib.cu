@@ -384,6 +384,7 @@ static int launch_point(fdfd_plan* P, const Geo<R>& g, const Op& op, RedBuf rb, 
 
 // ------------------------------------------------------------------ resident solves
 static constexpr int RES_CHUNK = 256;  // iterations per launch: a millisecond or two between polls
+static constexpr int RES_REFUSED = 1;  // the device does not take the cooperative launch; nothing ran
 
 // The brick split with the least work on the largest brick among those of at most one CTA
 // per SM that fit the shared memory with `nshell` shell vectors, one or two own cells per
@@ -424,13 +425,20 @@ static int launch_resident(fdfd_plan* P, void (*kern)(KArgs...), const ResidentP
   // (the attribute is set once per kernel: to the most any plan may ask for)
   if (int rc = ensure_smem(kern, P->smem_optin)) return rc;
   std::tuple<KArgs...> a(args...);
-  std::apply(
+  const cudaError_t e = std::apply(
       [&](auto&... v) {
         void* ptr[] = {(void*)&v...};
-        cudaLaunchCooperativeKernel((const void*)kern, dim3(rp.grid), dim3(RES_NT), ptr, rp.smem, s);
+        return cudaLaunchCooperativeKernel((const void*)kern, dim3(rp.grid), dim3(RES_NT), ptr, rp.smem, s);
       },
       a);
+  // a context may have fewer SMs than the device (an MPS share, a green context)
+  if (e == cudaErrorCooperativeLaunchTooLarge || e == cudaErrorLaunchOutOfResources || e == cudaErrorNotSupported ||
+      e == cudaErrorInvalidConfiguration) {
+    cudaGetLastError();
+    return RES_REFUSED;
+  }
   P->launches++;
+  CK(e);
   CKL();
   return 0;
 }
@@ -914,6 +922,9 @@ struct SolveCtx {
   unsigned long long tag;
   Word* surface;   // their surface words (two buffers of all cells), null: no room for them
   int limit;       // reads of a word before a CTA of theirs gives up
+  int launches_left;  // resident launches still allowed (negative: any number)
+  // One launch of theirs fewer; none once a wait ran out or a launch was refused.
+  bool take_launch() { return launches_left < 0 || launches_left-- > 0; }
   cx<double>* b;
   cx<double>* x;   // the caller's E
   cx<double>* e2;  // partner of E for the refinement ping-pong
@@ -961,6 +972,7 @@ static int refine_loop(SolveCtx& c, const Geo<RI>& gi, int prec, BsBufs B, doubl
     // ... or the inner precision is not enough for this problem: report it as a
     // breakdown so the caller can continue in complex128
     if (no_progress >= 2 || local_outer >= max_outer) { c.status = ST_BREAKDOWN; break; }
+    const double mon_before = prev_mon;
     prev_mon = mon;
     ++local_outer;
     ++c.outer;
@@ -993,20 +1005,23 @@ static int refine_loop(SolveCtx& c, const Geo<RI>& gi, int prec, BsBufs B, doubl
       return 0;
     };
     bool resident = false;
+    int rc = 0;
     if constexpr (sizeof(RI) == 4) {
       // As for COCG, every grid that fits runs resident.  r, t and x keep their vectors (t's
       // holds p between launches); the five between lie one after another and hold the
       // surface words (96 of their 120 bytes per cell).
-      resident = P->res_bs.grid > 0 && !P->profiling;
+      resident = P->res_bs.grid > 0 && !P->profiling && c.launches_left != 0;
       if (resident) {
         Word* surface = (Word*)B.R1;
         if (local_outer == 1) CK(cudaMemsetAsync(surface, 0, 5 * vb, s));
         const int nit = c.o->chunk > 0 ? c.o->chunk : RES_CHUNK;
-        TRY(drive(P, sti, nit, hi.maxiter, s, [&]() -> int {
+        rc = drive(P, sti, nit, hi.maxiter, s, [&]() -> int {
+          if (!c.take_launch()) return RES_REFUSED;
           const unsigned long long tag = c.tag;
           c.tag += (unsigned long long)nit;
           return launch_bicgstab_resident(P, (cx<RI>*)B.R0, (cx<RI>*)B.T, D, surface, seed, sti, c.scratch, tag, nit, c.limit, s);
-        }));
+        });
+        if (rc != 0 && rc != RES_REFUSED) return rc;
       }
     }
     // the shadow seed is baked into the batch, so graphs are keyed by it too
@@ -1023,8 +1038,17 @@ static int refine_loop(SolveCtx& c, const Geo<RI>& gi, int prec, BsBufs B, doubl
     }
     CK(cudaMemcpyAsync(P->h_state, sti, sizeof(KState), cudaMemcpyDeviceToHost, s));
     CK(cudaStreamSynchronize(s));
+    if (resident && (P->h_state->timed_out || (rc == RES_REFUSED && P->h_state->status == ST_RUNNING))) {
+      // what the SMs held is gone or does not belong together: this correction is formed
+      // again, from the field, by the two-launch form
+      c.launches_left = 0;
+      have_d = false;
+      prev_mon = mon_before;
+      --local_outer;
+      --c.outer;
+      continue;
+    }
     c.iters += P->h_state->iter;
-    if (P->h_state->timed_out) return set_err(FDFD_ERR_CUDA, "a CTA of a resident solve did not arrive in time");
     if (P->h_state->status == ST_NONFINITE) { c.status = ST_NONFINITE; break; }
     have_d = true;
   }
@@ -1078,20 +1102,35 @@ static int cocg_loop(SolveCtx& c, cx<double>* r, cx<double>* q, cx<double>* P0, 
   // Every grid that fits runs resident: it is 2 to 4 times faster than the two launches up to
   // the largest that do (52^3 and 380^2 cells, see k_cocg_resident).  The two-launch form
   // stays for larger grids, for profiling (which times its passes) and where the caller's
-  // workspace has no room for the surface words (the fallback of the mixed solver).
-  const bool resident = c.surface && P->res_cocg.grid > 0 && !P->profiling;
+  // workspace has no room for the surface words (the fallback of the mixed solver), and takes
+  // over where a cooperative launch is refused or a wait in one ran out.
+  bool resident = c.surface && P->res_cocg.grid > 0 && !P->profiling && c.launches_left != 0;
+  // A sequence started anew on the device counts on from c.iters: shift its cap and history.
+  auto count_on = [&]() -> int {
+    KState* hs = P->h_state;
+    CK(cudaMemcpyAsync(hs, st, sizeof(KState), cudaMemcpyDeviceToHost, s));
+    CK(cudaStreamSynchronize(s));
+    hs->maxiter = maxiter - c.iters;
+    hs->hist = o->history ? o->history + c.iters : nullptr;
+    hs->timed_out = 0;
+    CK(cudaMemcpyAsync(st, hs, sizeof(KState), cudaMemcpyHostToDevice, s));
+    return 0;
+  };
   int restarts = 0;
   for (;;) {
+    int rc = 0;
     CK(cudaMemcpyAsync(P->h_state, st, sizeof(KState), cudaMemcpyDeviceToHost, s));
     CK(cudaStreamSynchronize(s));
     const int left = maxiter - c.iters;
     if (resident && P->h_state->status == ST_RUNNING && left > 0) {
       const int nit = o->chunk > 0 ? o->chunk : RES_CHUNK;
-      TRY(drive(P, st, nit, left, s, [&]() -> int {
+      rc = drive(P, st, nit, left, s, [&]() -> int {
+        if (!c.take_launch()) return RES_REFUSED;
         const unsigned long long tag = c.tag;
         c.tag += (unsigned long long)nit;
         return launch_cocg_resident(P, r, P0, x, c.surface, st, c.scratch, tag, nit, c.limit, s);
-      }));
+      });
+      if (rc != 0 && rc != RES_REFUSED) return rc;
     } else if (P->h_state->status == ST_RUNNING && left > 0) {
       TRY(drive(P, st, chunk, left, s, [&]() -> int {
         if (o->use_graph && !P->profiling) {
@@ -1107,9 +1146,21 @@ static int cocg_loop(SolveCtx& c, cx<double>* r, cx<double>* q, cx<double>* P0, 
     }
     CK(cudaMemcpyAsync(P->h_state, st, sizeof(KState), cudaMemcpyDeviceToHost, s));
     CK(cudaStreamSynchronize(s));
+    if (resident && (P->h_state->timed_out || (rc == RES_REFUSED && P->h_state->status == ST_RUNNING))) {
+      // The bricks may be a step apart, but any field is one to go on from: its residual, and
+      // the two-launch form.  A step that not all CTAs took does not count.
+      const int lost = P->h_state->timed_out && P->h_state->status != ST_TIMEOUT;
+      c.iters += std::max(0, P->h_state->iter - lost);
+      c.launches_left = 0;
+      resident = false;
+      OpCocgInit<double> op{c.b, x, r, N, st, 0.0, 0U, nullptr};
+      TRY(launch_stencil<double>(P, P->g64, 0, op, rb, s));
+      CK(cudaMemsetAsync(P0, 0, vbytes128, s));
+      TRY(count_on());
+      continue;
+    }
     c.iters += P->h_state->iter;
     c.status = P->h_state->status;
-    if (P->h_state->timed_out) return set_err(FDFD_ERR_CUDA, "a CTA of a resident solve did not arrive in time");
     if (c.status == ST_RUNNING) c.status = ST_MAXITER;
     if (c.status != ST_BREAKDOWN || restarts >= 8 || c.iters >= maxiter) break;
     // Breakdown: the unconjugated form cancelled (for example a source whose
@@ -1132,13 +1183,7 @@ static int cocg_loop(SolveCtx& c, cx<double>* r, cx<double>* q, cx<double>* P0, 
     }
     CK(cudaMemcpyAsync(x, c.e2, vbytes128, cudaMemcpyDeviceToDevice, s));
     CK(cudaMemsetAsync(P0, 0, vbytes128, s));
-    // the restarted sequence counts on from c.iters: shift its cap and history
-    KState* hs = P->h_state;
-    CK(cudaMemcpyAsync(hs, st, sizeof(KState), cudaMemcpyDeviceToHost, s));
-    CK(cudaStreamSynchronize(s));
-    hs->maxiter = maxiter - c.iters;
-    hs->hist = o->history ? o->history + c.iters : nullptr;
-    CK(cudaMemcpyAsync(st, hs, sizeof(KState), cudaMemcpyHostToDevice, s));
+    TRY(count_on());
   }
   if (c.status == ST_BREAKDOWN || c.status == ST_NONFINITE) {
     // still stuck: continue from the current iterate with complex128 BiCGSTAB
@@ -1182,6 +1227,7 @@ extern "C" int fdfd_solve(fdfd_plan* P, const fdfd_solve_opts* o, const void* J,
   c.tag = 0;
   c.surface = nullptr;
   c.limit = o->wait_limit > 0 ? o->wait_limit : SPIN_LIMIT;
+  c.launches_left = o->wait_limit < 0 ? -(o->wait_limit + 1) : -1;
   c.b = (cx<double>*)(base + L.b);
   c.x = (cx<double>*)E;
   c.e2 = (cx<double>*)(base + L.e2);

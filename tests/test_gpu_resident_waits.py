@@ -60,3 +60,30 @@ def test_a_converged_field_has_no_stale_brick(problem):
                     continue
                 # the residual is formed again from the field at the end
                 assert info.converged and info.residual <= 1.0001 * rtol, limit
+
+
+@pytest.mark.parametrize('limit', [-1, -2, -3, -20, 1, 3, 5, 10, 20])
+@pytest.mark.parametrize('chunk', [1, 3, 0])
+@pytest.mark.parametrize('method,adjoint', [('cocg', False), ('cocg', True), ('mixed', False)])
+def test_the_solve_goes_on_without_the_resident_form(problem, method, adjoint, chunk, limit):
+    """A wait that runs out, or no (further) resident launch: no error, the same solution, the
+    cap on the iterations and a history without gaps."""
+    op, J = problem
+    kw = dict(method=method, rtol=1e-11, criterion='true', chunk=chunk, adjoint=adjoint, maxiter=4000)
+    ref, _ = op.solve(J, **kw)
+    for _ in range(3):
+        E, info = op.solve(J, wait_limit=limit, record_history=method == 'cocg', **kw)
+        assert info.converged and info.residual <= 1.01e-11 and info.iterations <= 4000
+        assert float((E - ref).norm()) <= 1e-7 * float(ref.norm())
+        if method == 'cocg':
+            assert numpy.all(info.history[1:] > 0) and info.history[-1] <= 1e-11
+    again, _ = op.solve(J, **kw)
+    assert numpy.array_equal(again.cpu().numpy(), ref.cpu().numpy())
+
+
+@pytest.mark.parametrize('limit', [0, -1, -4, 2, 6])
+def test_the_cap_holds_when_the_form_changes(problem, limit):
+    op, J = problem
+    E, info = op.solve(J, rtol=1e-13, criterion='true', chunk=1, maxiter=7, wait_limit=limit)
+    assert (info.status, info.iterations) == ('maxiter', 7)
+    assert abs(op.residual(E, J)['rel'] / info.residual - 1) <= 1e-9
