@@ -160,25 +160,37 @@ __device__ __forceinline__ bool sums_end(double* out, int* gave_up, ResidentScra
   return *gave_up == 0;
 }
 
-// 1 / d for d in [1, 8): the hardware's approximate reciprocal (better than 2^-20) and two
-// Newton steps, whose errors square (2^-40, then rounding): within an ulp or two.  A full
-// division is some 400 cycles of latency, an iteration's scalar work had six of them.
+// x / d for normal d, from the hardware's approximate reciprocal (better than 2^-20), two
+// Newton steps, whose errors square (2^-40, then rounding: within an ulp), and the residual of
+// the quotient, which rounds it as a division does but for rare last bits.  A division is some
+// 400 cycles of latency, an iteration's scalar work had six to nine of them.
 __device__ __forceinline__ double newton_reciprocal(double d) {
   double y;
   asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(d));
   y = fma(y, fma(-d, y, 1.0), y);
   return fma(y, fma(-d, y, 1.0), y);
 }
+__device__ __forceinline__ double quotient(double x, double d, double inv_d) {
+  const double q = x * inv_d;
+  return fma(fma(-q, d, x), inv_d, q);
+}
 
-// a / b: b scaled by a power of two so that |b|^2 is in [1, 8).
+// a / b by Smith's algorithm as in ddiv, with quotients of that kind, where the exponents keep
+// them far from overflow and underflow (|a| and |b| within 2^+-450); ddiv elsewhere.  Largest
+// and root mean square error over random pairs, in units of 2^-53 |a / b|: 2.9 and 0.75, as
+// ddiv's (a conj(b) / |b|^2 with the same reciprocals: 4.6 and 0.95).
+__device__ __forceinline__ bool mid_range(dcx z) {
+  const int e = (__double2hiint(fmax(fabs(z.re), fabs(z.im))) >> 20) & 0x7ff;
+  return (unsigned)(e - 573) <= 900u;
+}
 __device__ __forceinline__ dcx cdiv(dcx a, dcx b) {
-  const double big = fmax(fabs(b.re), fabs(b.im));
-  const int e = (__double2hiint(big) >> 20) & 0x7ff;
-  if (e < 24 || e > 2022) return ddiv(a, b);
-  const double sc = __hiloint2double((2046 - e) << 20, 0);  // 2^(1023 - e): big * sc in [1, 2)
-  const double re = b.re * sc, im = b.im * sc;
-  const double inv = sc * newton_reciprocal(fma(re, re, im * im));
-  return {fma(a.re, re, a.im * im) * inv, fma(a.im, re, -(a.re * im)) * inv};
+  if (!mid_range(a) || !mid_range(b)) return ddiv(a, b);
+  const bool swap = fabs(b.re) < fabs(b.im);
+  const double p = swap ? b.im : b.re, o = swap ? b.re : b.im;
+  const double r = quotient(o, p, newton_reciprocal(p)), d = fma(o, r, p), inv_d = newton_reciprocal(d);
+  const double re = swap ? fma(a.re, r, a.im) : fma(a.im, r, a.re);
+  const double im = swap ? fma(a.im, r, -a.re) : fma(-a.re, r, a.im);
+  return {quotient(re, d, inv_d), quotient(im, d, inv_d)};
 }
 
 // The three components at a surface cell, rows of n words (complex128: one row per real
@@ -529,7 +541,7 @@ __host__ __device__ inline ResidentLayout resident_layout(int nshell, int nred, 
 // Measured per iteration, two launches / resident: 16^3 25.0 / 5.9 us, 40^3 28.5 / 9.9, 52^3
 // (the largest cube that fits) 37.4 / 16.9; flat 128^2 23.4 / 6.1, 380^2 34.2 / 11.0.  It is
 // bound by the exchanges (about 3 us of each iteration) and, on full bricks, by shared-memory
-// bandwidth in the two curl passes.  Of that, dividing by newton_reciprocal, block sums through
+// bandwidth in the two curl passes.  Of that, dividing by reciprocals (cdiv), block sums through
 // shared memory and material code by template gave 0.4 to 0.8 us.
 constexpr int COCG_SUMS = 5;
 template <int NT, int K, bool FLAT, bool MAT>
@@ -932,10 +944,22 @@ __global__ void __launch_bounds__(NT, 1)
       break;
     }
     const bool small_s = ss <= tol2 || tt <= 0.0;  // s small enough (or t vanished): finish with omega = 0
-    const double itt = small_s ? 0.0 : 1.0 / tt;
-    const dcx om = {ts.re * itt, ts.im * itt};
+    dcx om = {0.0, 0.0};
+    rr = ss;
+    if (!small_s) {
+      const double tstt = ts.re * ts.re + ts.im * ts.im;
+      double off;  // |(t, s)|^2 / |t|^2
+      if (mid_range(ts) && mid_range({tt, 0.0})) {
+        const double itt = newton_reciprocal(tt);
+        om = {quotient(ts.re, tt, itt), quotient(ts.im, tt, itt)};
+        off = quotient(tstt, tt, itt);
+      } else {
+        om = {ts.re / tt, ts.im / tt};
+        off = tstt / tt;
+      }
+      rr = fmax(ss - off, 0.0);
+    }
     omega = from_d<R>(om);
-    rr = small_s ? ss : fmax(ss - (ts.re * ts.re + ts.im * ts.im) * itt, 0.0);
     if (rr <= tol2) status = ST_CONVERGED;
     else if (iter >= maxiter) status = ST_MAXITER;
     if (status == ST_RUNNING && small_s) status = ST_BREAKDOWN;
