@@ -111,7 +111,7 @@ struct Tiling {
 // grid does not fit).
 struct ResidentPlan {
   Bricks bk;
-  int k, grid;
+  int k, grid, nt;
   size_t smem;
 };
 
@@ -386,12 +386,12 @@ static int launch_point(fdfd_plan* P, const Geo<R>& g, const Op& op, RedBuf rb, 
 static constexpr int RES_CHUNK = 256;  // iterations per launch: a millisecond or two between polls
 static constexpr int RES_REFUSED = 1;  // the device does not take the cooperative launch; nothing ran
 
-// The brick split with the least work on the largest brick among those of at most one CTA
-// per SM that fit the shared memory with `nshell` shell vectors, one or two own cells per
-// thread.  Work: an own cell takes part in every pass, a shell cell and an H cell in one or
-// two.
+// The brick split with the least work on the largest brick among those of at most one CTA of
+// `nt` threads per SM that fit the shared memory with `nshell` shell vectors, at most `kmax`
+// (1 or 2) own cells per thread.  Work: an own cell takes part in every pass, a shell cell and
+// an H cell in one or two.
 template <typename R>
-static ResidentPlan plan_resident(const fdfd_plan* P, int nshell, int nred, size_t smem_max) {
+static ResidentPlan split_bricks(const fdfd_plan* P, int nshell, int nred, int nt, int kmax, size_t smem_max) {
   ResidentPlan best{};
   long long best_cost = -1;
   const int most = std::min(P->nsm, RES_CTAS);
@@ -400,23 +400,36 @@ static ResidentPlan plan_resident(const fdfd_plan* P, int nshell, int nred, size
       for (int nz = 1; nz <= (P->flat ? 1 : std::min(P->Z, most / (nx * ny))); ++nz) {
         const int bx = (P->X + nx - 1) / nx, by = (P->Y + ny - 1) / ny, bz = (P->Z + nz - 1) / nz;
         const long long own = (long long)bx * by * bz;
-        int k = 1;
-        if (own > RES_NT) k = 2;
-        if ((long long)((bx + k - 1) / k) * by * bz > RES_NT) continue;
+        const int k = own > nt ? 2 : 1;
+        if (k > kmax || (long long)((bx + k - 1) / k) * by * bz > nt) continue;
         const int kz = P->flat ? 0 : 1;
         const long long box = (long long)(bx + 2) * (by + 2) * (bz + 2 * kz);
         const long long hbox = (long long)(bx + 1) * (by + 1) * (bz + kz);
-        const size_t smem = resident_layout<R>(nshell, nred, P->flat, bx, by, bz).total;
+        const size_t smem = resident_layout<R>(nshell, nred, P->flat, bx, by, bz, nt).total;
         if (smem > smem_max) continue;
         const long long cost = own + box + hbox;
         if (best_cost < 0 || cost < best_cost) {
           best_cost = cost;
-          best = ResidentPlan{Bricks{nx, ny, nz, bx, by, bz}, k, nx * ny * nz, smem};
+          best = ResidentPlan{Bricks{nx, ny, nz, bx, by, bz}, k, nx * ny * nz, nt, smem};
         }
       }
     }
   }
   return best;
+}
+
+// CTAs of half an SM where bricks of one cell per thread (two on flat grids) cover the grid,
+// otherwise of a whole SM.  A launch of the latter has the GPU to itself for its 256
+// iterations, so solves on other streams take turns with it, while two of the former share the
+// SMs.  Alone / eight at once, us per iteration of the two-launch form before, whole SM, half:
+// BiCGSTAB 128x128 30 / 4.7, 6.6 / 6.3, 6.4 / 3.4; 256x256 32 / 6.6, 7.6 / 7.3, 8.1 / 5.0; COCG 24^3
+// 26 / 3.9, 6.3 / 6.0, 6.1 / 3.4; 32^3 27 / 4.7, 7.7 / 7.4, 7.5 / 5.0.  Larger 3D grids gain on whole SMs
+// either way: 36^3 29 / 9.2, 8.2 / 7.9, 11.3 / 6.9 (two cells per thread); 48^3 31 / 16, 12.4 / 12.2, does
+// not fit.
+template <typename R>
+static ResidentPlan plan_resident(const fdfd_plan* P, int nshell, int nred, size_t smem_max, size_t smem_half) {
+  const ResidentPlan half = split_bricks<R>(P, nshell, nred, RES_NT_HALF, P->flat ? 2 : 1, smem_half);
+  return half.grid > 0 ? half : split_bricks<R>(P, nshell, nred, RES_NT, 2, smem_max);
 }
 
 template <class... KArgs, class... Args>
@@ -428,7 +441,7 @@ static int launch_resident(fdfd_plan* P, void (*kern)(KArgs...), const ResidentP
   const cudaError_t e = std::apply(
       [&](auto&... v) {
         void* ptr[] = {(void*)&v...};
-        return cudaLaunchCooperativeKernel((const void*)kern, dim3(rp.grid), dim3(RES_NT), ptr, rp.smem, s);
+        return cudaLaunchCooperativeKernel((const void*)kern, dim3(rp.grid), dim3(rp.nt), ptr, rp.smem, s);
       },
       a);
   // a context may have fewer SMs than the device (an MPS share, a green context)
@@ -443,18 +456,21 @@ static int launch_resident(fdfd_plan* P, void (*kern)(KArgs...), const ResidentP
   return 0;
 }
 
-// The instance of a resident kernel for a plan: cells per thread, flat, materials.
-#define RES_PICK(name, k, flat, mat)                                                                              \
-  ((k) == 1 ? ((flat) ? ((mat) ? name<RES_NT, 1, true, true> : name<RES_NT, 1, true, false>)                      \
-                      : ((mat) ? name<RES_NT, 1, false, true> : name<RES_NT, 1, false, false>))                   \
-            : ((flat) ? ((mat) ? name<RES_NT, 2, true, true> : name<RES_NT, 2, true, false>)                      \
-                      : ((mat) ? name<RES_NT, 2, false, true> : name<RES_NT, 2, false, false>)))
+// The instance of a resident kernel for a plan: threads, cells per thread, flat, materials (of
+// the combinations that plan_resident makes).
+#define RES_MAT(name, nt, k, flat, mat) ((mat) ? name<nt, k, flat, true> : name<nt, k, flat, false>)
+#define RES_PICK(name, rp, flat, mat)                                                                      \
+  ((rp).nt == RES_NT_HALF                                                                                  \
+       ? ((flat) ? ((rp).k == 1 ? RES_MAT(name, RES_NT_HALF, 1, true, mat) : RES_MAT(name, RES_NT_HALF, 2, true, mat)) \
+                 : RES_MAT(name, RES_NT_HALF, 1, false, mat))                                              \
+       : ((flat) ? RES_MAT(name, RES_NT, 2, true, mat)                                                     \
+                 : ((rp).k == 1 ? RES_MAT(name, RES_NT, 1, false, mat) : RES_MAT(name, RES_NT, 2, false, mat))))
 
 static int launch_cocg_resident(fdfd_plan* P, cx<double>* r, cx<double>* p, cx<double>* x, Word* surface, KState* st,
                                 ResidentScratch* gs, unsigned long long tag, int nit, int limit, cudaStream_t s) {
   const ResidentPlan& rp = P->res_cocg;
   CK(cudaMemsetAsync(gs->counter, 0, sizeof(gs->counter), s));
-  return launch_resident(P, RES_PICK(k_cocg_resident, rp.k, P->flat, P->has_mu || P->has_mask), rp, s, P->g64, rp.bk, r,
+  return launch_resident(P, RES_PICK(k_cocg_resident, rp, P->flat, P->has_mu || P->has_mask), rp, s, P->g64, rp.bk, r,
                          p, x, surface, st, gs, tag, nit, limit);
 }
 
@@ -463,7 +479,7 @@ static int launch_bicgstab_resident(fdfd_plan* P, cx<float>* r, cx<float>* p, cx
                                     int limit, cudaStream_t s) {
   const ResidentPlan& rp = P->res_bs;
   CK(cudaMemsetAsync(gs->counter, 0, sizeof(gs->counter), s));
-  return launch_resident(P, RES_PICK(k_bicgstab_resident, rp.k, P->flat, P->has_mu || P->has_mask), rp, s, P->g32, rp.bk,
+  return launch_resident(P, RES_PICK(k_bicgstab_resident, rp, P->flat, P->has_mu || P->has_mask), rp, s, P->g32, rp.bk,
                          r, p, x, surface, seed, st, gs, tag, nit, limit);
 }
 
@@ -634,13 +650,16 @@ extern "C" int fdfd_plan_create(const fdfd_grid_desc* d, void* ws, size_t ws_byt
   cudaDeviceGetAttribute(&P->nsm, cudaDevAttrMultiProcessorCount, dev);
   if (P->nsm <= 0) P->nsm = 148;
   {
-    int coop = 0, optin = 0;
+    int coop = 0, optin = 0, per_sm = 0, reserved = 0;
     cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, dev);
     cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev);
+    cudaDeviceGetAttribute(&per_sm, cudaDevAttrMaxSharedMemoryPerMultiprocessor, dev);
+    cudaDeviceGetAttribute(&reserved, cudaDevAttrReservedSharedMemoryPerBlock, dev);
     P->smem_optin = (size_t)optin;
+    const size_t half = (size_t)std::max(0, per_sm / 2 - reserved);
     if (coop) {
-      P->res_cocg = plan_resident<double>(P, 1, COCG_SUMS, P->smem_optin);
-      if (P->has32) P->res_bs = plan_resident<float>(P, 4, BS_SUMS, P->smem_optin);
+      P->res_cocg = plan_resident<double>(P, 1, COCG_SUMS, P->smem_optin, half);
+      if (P->has32) P->res_bs = plan_resident<float>(P, 4, BS_SUMS, P->smem_optin, half);
     }
   }
   auto cleanup = [&](int rc) {

@@ -237,6 +237,19 @@ __device__ __forceinline__ bool surface_load(const Word* w, size_t n, int cell, 
   return ok;
 }
 
+// Which entries of the shell list a thread reads while NRED warps wait for sums: where those
+// are less than half of the CTA they read none, otherwise they come last (32^3 with 256
+// threads, none / last: COCG 8.2 / 7.6 us per iteration, BiCGSTAB 9.3 / 8.6).
+template <int NT, int NRED>
+struct ShellReaders {
+  static constexpr int waiting = 32 * NRED;
+  static constexpr bool all = 2 * waiting > NT;
+  static constexpr int step = all ? NT : NT - waiting;
+  static __device__ __forceinline__ int first(int tid) {  // (negative: none)
+    return all && tid < waiting ? tid - waiting + NT : tid - waiting;
+  }
+};
+
 // Whether a launch has work.  One thread looks and the CTA follows: a CTA may start while
 // others give up already.
 __device__ __forceinline__ bool resident_begin(KState* st) {
@@ -511,9 +524,12 @@ __device__ __forceinline__ void list_shell(const Geo<R>& g, const Brick<R, FLAT>
 struct ResidentLayout {
   size_t shell_vec, h, shell, tables, red, total;
 };
-constexpr int RES_NT = 512;  // threads: 128 registers each (576 to 768 threads spill more and are slower)
+// Threads of a CTA, of 128 registers each: a whole SM's (576 to 768 spill more and are slower),
+// or half of them, so that two solves can share the SMs (see plan_resident).
+constexpr int RES_NT = 512, RES_NT_HALF = 256;
 template <typename R>
-__host__ __device__ inline ResidentLayout resident_layout(int nshell, int nred, bool flat, int bx, int by, int bz) {
+__host__ __device__ inline ResidentLayout resident_layout(int nshell, int nred, bool flat, int bx, int by, int bz,
+                                                          int nt) {
   const size_t kz = flat ? 0 : 1;
   const size_t box = (size_t)(bx + 2) * (by + 2) * (bz + 2 * kz), own = (size_t)bx * by * bz;
   const size_t hbox = (size_t)(bx + 1) * (by + 1) * (bz + kz);
@@ -523,7 +539,7 @@ __host__ __device__ inline ResidentLayout resident_layout(int nshell, int nred, 
   L.shell = (L.h + sizeof(cx<R>) * 3 * hbox + 15) & ~(size_t)15;
   L.tables = L.shell + ((sizeof(int2) * (box - own) + 15) & ~(size_t)15);
   L.red = L.tables + ((BrickTables<R>::bytes(bx, by, bz) + 15) & ~(size_t)15);
-  L.total = L.red + ((size_t)nred * RedRow<RES_NT>::value + 2 * RES_SUMS + 2) * sizeof(double);
+  L.total = L.red + ((size_t)nred * (nt / 4) + 2 * RES_SUMS + 2) * sizeof(double);
   return L;
 }
 
@@ -545,14 +561,14 @@ __host__ __device__ inline ResidentLayout resident_layout(int nshell, int nred, 
 // shared memory and material code by template gave 0.4 to 0.8 us.
 constexpr int COCG_SUMS = 5;
 template <int NT, int K, bool FLAT, bool MAT>
-__global__ void __launch_bounds__(NT, 1)
+__global__ void __launch_bounds__(NT, RES_NT / NT)
     k_cocg_resident(const Geo<double> g, const Bricks bk, cx<double>* r, cx<double>* p, cx<double>* x, Word* surface,
                     KState* st, ResidentScratch* gs, unsigned long long tag0, int nit, int limit) {
   using R = double;
   using C = cx<R>;
   if (!resident_begin(st)) return;
   extern __shared__ __align__(16) unsigned char smem_raw[];
-  const ResidentLayout L = resident_layout<R>(1, COCG_SUMS, FLAT, bk.bx, bk.by, bk.bz);
+  const ResidentLayout L = resident_layout<R>(1, COCG_SUMS, FLAT, bk.bx, bk.by, bk.bz, NT);
   Brick<R, FLAT> B;
   B.init(g, bk);
   C* P = reinterpret_cast<C*>(smem_raw);
@@ -685,15 +701,15 @@ __global__ void __launch_bounds__(NT, 1)
       }
       sums_begin<NT, 2, NRHO>(acc, red, gs, tag);
     }
-    // while the sums travel: the loads of x, and the shell's r in the warps that do not wait
-    // for a sum
+    // while the sums travel: the loads of x, and the shell's r
 #pragma unroll
     for (int m = 0; m < K; ++m) {
       if (m >= o.n) break;
 #pragma unroll
       for (int c = 0; c < 3; ++c) t[m][c] = x[c * N + o.cell + m * YZ];
     }
-    for (int e = tid - 32 * NRHO; e >= 0 && e < nshell; e += NT - 32 * NRHO) {
+    using Readers = ShellReaders<NT, NRHO>;
+    for (int e = Readers::first(tid); e >= 0 && e < nshell; e += Readers::step) {
       C qv[3];
       if (!surface_load<R>(sw, (size_t)N, shell[e].y, qv, tag, limit)) flags[1] = 1;
 #pragma unroll
@@ -775,7 +791,7 @@ __global__ void __launch_bounds__(NT, 1)
 // Bound as COCG is: two exchanges, then shared-memory bandwidth on full bricks.
 constexpr int BS_SUMS = 6;
 template <int NT, int K, bool FLAT, bool MAT>
-__global__ void __launch_bounds__(NT, 1)
+__global__ void __launch_bounds__(NT, RES_NT / NT)
     k_bicgstab_resident(const Geo<float> g, const Bricks bk, cx<float>* r, cx<float>* p, cx<float>* x, Word* surface,
                         unsigned seed, KState* st, ResidentScratch* gs, unsigned long long tag0, int nit,
                         int limit) {
@@ -783,7 +799,7 @@ __global__ void __launch_bounds__(NT, 1)
   using C = cx<R>;
   if (!resident_begin(st)) return;
   extern __shared__ __align__(16) unsigned char smem_raw[];
-  const ResidentLayout L = resident_layout<R>(4, BS_SUMS, FLAT, bk.bx, bk.by, bk.bz);
+  const ResidentLayout L = resident_layout<R>(4, BS_SUMS, FLAT, bk.bx, bk.by, bk.bz, NT);
   Brick<R, FLAT> B;
   B.init(g, bk);
   C* U = reinterpret_cast<C*>(smem_raw);
@@ -871,8 +887,8 @@ __global__ void __launch_bounds__(NT, 1)
       double acc[NS] = {(double)a[0], (double)a[1]};
       sums_begin<NT, 0, NS>(acc, red, gs, tag);
     }
-    // while the sums travel: v of the shell, in the warps that do not wait for a sum
-    for (int e = tid - 32 * NS; e >= 0 && e < nshell; e += NT - 32 * NS) {
+    // while the sums travel: v of the shell
+    for (int e = ShellReaders<NT, NS>::first(tid); e >= 0 && e < nshell; e += ShellReaders<NT, NS>::step) {
       C q[3];
       if (!surface_load<R>(surface, nw, shell[e].y, q, tag, it > 0 ? limit : SPIN_LIMIT)) flags[1] = 1;
 #pragma unroll
@@ -928,7 +944,7 @@ __global__ void __launch_bounds__(NT, 1)
       for (int q = 0; q < NT6; ++q) acc[q] = (double)a[q];
       sums_begin<NT, NS, NT6>(acc, red, gs, tag);
     }
-    for (int e = tid - 32 * NT6; e >= 0 && e < nshell; e += NT - 32 * NT6) {
+    for (int e = ShellReaders<NT, NT6>::first(tid); e >= 0 && e < nshell; e += ShellReaders<NT, NT6>::step) {
       C q[3];
       if (!surface_load<R>(surface + SurfaceRows<R>::value * nw, nw, shell[e].y, q, tag, limit)) flags[1] = 1;
 #pragma unroll
