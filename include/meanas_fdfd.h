@@ -94,8 +94,8 @@ typedef struct fdfd_solve_opts {
   int32_t max_outer;     /* MIXED: refinement steps cap (0 = default)               */
   double inner_rtol;     /* MIXED: residual reduction per inner solve (0 = default) */
   double* history;       /* optional device float64[maxiter + 1]: relative residuals */
-  int32_t profile;       /* nonzero: time every iteration kernel with CUDA events (no
-                            graphs); fills the *_ms / *_launches fields of the info  */
+  int32_t profile;       /* nonzero: time every iteration kernel with CUDA events (a launch per
+                            pass: no graphs, not resident); fills kernel_ms / kernel_count */
   int32_t wait_limit;    /* reads of a word after which a CTA of a resident solve stops waiting for
                             the others and the solve goes on with a launch per pass (0 =
                             default, one to two seconds); -n: after n - 1 resident launches */
@@ -143,6 +143,12 @@ int fdfd_plan_destroy(fdfd_plan* plan);
 
 /* Override the x-planes-per-CTA tiling for one precision (autotuner hook). */
 int fdfd_plan_set_xchunk(fdfd_plan* plan, int32_t precision, int32_t xchunk);
+
+/* Whether fdfd_solve runs this plan's grid resident with `method`: the CTAs of the cooperative
+ * launch that keeps the Krylov vectors on the SMs for many iterations, or 0 when every pass is
+ * a launch (grids that do not fit, FDFD_METHOD_BICGSTAB).  The tiling above does not matter to
+ * the iterations of resident solves. */
+int fdfd_plan_resident(const fdfd_plan* plan, int32_t method);
 
 /* Matrix-free operator product y = op(x) in complex128 or complex64 (x, y: 3N).
  * FDFD_OP_A0 replaces operators.e_full(...) @ x (meanas/fdfd/operators.py:40-96);

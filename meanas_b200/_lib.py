@@ -107,6 +107,7 @@ EXPORTS = {
     'fdfd_plan_update': (C.c_int, [C.c_void_p, C.POINTER(GridDesc), C.c_void_p]),
     'fdfd_plan_destroy': (C.c_int, [C.c_void_p]),
     'fdfd_plan_set_xchunk': (C.c_int, [C.c_void_p, C.c_int32, C.c_int32]),
+    'fdfd_plan_resident': (C.c_int, [C.c_void_p, C.c_int32]),
     'fdfd_apply': (C.c_int, [C.c_void_p, C.c_int32, C.c_int32, C.c_void_p, C.c_void_p, C.c_void_p]),
     'fdfd_solve_workspace_bytes': (C.c_int, [C.c_void_p, C.POINTER(SolveOpts), C.POINTER(C.c_size_t)]),
     'fdfd_solve': (C.c_int, [C.c_void_p, C.POINTER(SolveOpts), C.c_void_p, C.c_void_p, C.c_void_p, C.c_size_t,

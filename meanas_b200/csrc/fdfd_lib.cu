@@ -728,6 +728,12 @@ extern "C" int fdfd_plan_set_xchunk(fdfd_plan* P, int32_t precision, int32_t xch
   return 0;
 }
 
+extern "C" int fdfd_plan_resident(const fdfd_plan* P, int32_t method) {
+  if (!P || method < FDFD_METHOD_COCG || method > FDFD_METHOD_BICGSTAB)
+    return set_err(FDFD_ERR_ARG, "bad arguments to fdfd_plan_resident");
+  return method == FDFD_METHOD_COCG ? P->res_cocg.grid : (method == FDFD_METHOD_MIXED ? P->res_bs.grid : 0);
+}
+
 // ------------------------------------------------------------------ apply
 extern "C" int fdfd_apply(fdfd_plan* P, int32_t op, int32_t precision, const void* x, void* y, void* stream) {
   if (!P || !x || !y) return set_err(FDFD_ERR_ARG, "fdfd_apply: NULL argument");

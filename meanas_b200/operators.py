@@ -199,6 +199,11 @@ class GridOperator:
         0 restores the default."""
         _lib.check(self.lib.fdfd_plan_set_xchunk(self.plan, _PREC[precision], int(xchunk)))
 
+    def resident(self, method: str = 'cocg') -> bool:
+        """Whether solves with ``method`` keep the Krylov vectors on the SMs (grids of up to about
+        52^3 or 380^2 cells).  The x chunk does not matter to their iterations."""
+        return _lib.check(self.lib.fdfd_plan_resident(self.plan, _METHODS[method])) > 0
+
     # ------------------------------------------------------------------ products
     def apply(self, x, op: str = 'A0', precision: str = 'c128', out: torch.Tensor | None = None) -> torch.Tensor:
         """``y = op(x)``: ``'A0'``, ``'sym'`` (Pl A0 Pr) or ``'sym_h'`` ((Pl A0 Pr)^H)."""
@@ -317,7 +322,9 @@ class GridOperator:
         ``iters`` iterations of the real solver passes on dense data (a random initial
         guess), with per-kernel CUDA events; the figure compared is the median of three
         such runs.  The choice is kept for the process: later operators of the same grid
-        size on the same device start from it.  Returns {precision: (xchunk, us/iteration, all)}."""
+        size on the same device start from it.  Where solves run resident (``resident``) the
+        passes timed here serve profiling, the mixed solver's fallback and, by the same
+        tiling, products only.  Returns {precision: (xchunk, us/iteration, all)}."""
         X = self.shape[0]
         cands = {}
         if candidates is None:

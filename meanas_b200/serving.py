@@ -5,16 +5,18 @@ return futures.  The server keeps **slots**: device-resident solver state for on
 size (a ``GridOperator`` with its plan, the solve workspace with the Krylov vectors,
 the field buffer and a CUDA stream).  A slot serves request after request of its size:
 a new request is copied into the slot's buffers and the plan is refilled in place
-(``fdfd_plan_update``), so the iteration bodies captured as CUDA graphs for that size
-are replayed, not re-captured.
+(``fdfd_plan_update``), so for grids too large to run resident the iteration bodies
+captured as CUDA graphs for that size are replayed, not re-captured.
 
 Admission: a worker picks the oldest waiting request whose slot (idle, or new within
 the HBM budget) is available; idle slots of other sizes are released when the budget
 needs room.  Up to ``max_active`` solves run at once, each on its own stream and
 host thread (the C call releases the GIL), so requests that arrive while others are
-on the GPU start as soon as a slot and memory free up and their kernels overlap on
-the device.  Every solve is deterministic (fixed-order reductions, fixed tiling per
-slot), so a request's result does not depend on what else is in flight.
+on the GPU start as soon as a slot and memory free up.  Small grids (up to about 33^3 or
+270^2 cells) run resident on half of every SM, two at a time; resident solves up to
+about 52^3 or 380^2 take turns at whole SMs; the kernels of larger ones overlap.  Every
+solve is deterministic (fixed-order reductions, fixed tiling per slot), so a request's
+result does not depend on what else is in flight.
 """
 from __future__ import annotations
 
@@ -88,8 +90,9 @@ class _Slot:
             if xchunk:
                 self.op.set_xchunk(prec, xchunk)
                 self.xchunk = xchunk
-            elif autotune:
-                # the first slot of a size times the x-chunk candidates on its own stream
+            elif autotune and not self.op.resident('mixed' if precision == 'mixed' else 'cocg'):
+                # the first slot of a size times the x-chunk candidates on its own stream (the
+                # iterations of a resident solve have none)
                 key = (self.op.device.index, tuple(shape), prec)
                 with _TUNE_GUARD:
                     lock = _TUNE_LOCKS[key]
@@ -119,9 +122,9 @@ class FDFDServer:
     the slots may hold (default: 80 % of free memory at start-up).  ``precision``:
     ``'mixed'`` (complex64 BiCGSTAB + complex128 refinement) or ``'fp64'`` (COCG).
     ``rtol``: true FP64 residual target.  ``xchunk``: optional fixed x planes per CTA;
-    otherwise (``autotune=True``) the first slot of each grid size times the candidates
-    (``GridOperator.autotune``) and every later slot of that size reuses the choice, or
-    (``autotune=False``) the library's default.
+    otherwise (``autotune=True``) the first slot of each grid size too large to run resident
+    times the candidates (``GridOperator.autotune``) and every later slot of that size reuses
+    the choice, or (``autotune=False``) the library's default.
     """
 
     def __init__(self, device: Any | None = None, *, max_active: int = 8, hbm_budget: int | None = None,
