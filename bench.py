@@ -76,6 +76,7 @@ def kernel_bytes(kind: int, p) -> int:
 
 
 METHOD_NAMES = {'cocg': 'fp64 (complex128 COCG)', 'mixed': 'mixed (complex64 inner, complex128 refinement)'}
+RESIDENT_NAMES = {'cocg': 'cocg_resident_c128', 'mixed': 'bicgstab_resident_c64'}
 KERNEL_NAMES = {0: 'cocg_stencil_c128', 1: 'cocg_point_c128', 2: 'bicgstab_P_c64', 3: 'bicgstab_S_c64'}
 
 
@@ -92,15 +93,17 @@ def peaks() -> tuple[float, str]:
 PROFILE_TAGS = {'aniso_blocks': 'aniso160', 'dipole_core': 'dipole48', 'masked_large': 'masked320'}
 
 
-def profile_traffic(kernel: str, workload: str) -> tuple[float | None, str | None]:
+def profile_traffic(kernel: str, workload: str, average: bool = False) -> tuple[float | None, str | None]:
     """DRAM bytes per launch of `kernel` on `workload` from the committed ncu summary
     profiles/<kernel>_<workload tag>.md, and where that number comes from (the file and the
-    source commit it records for the capture).  (None, None) when no capture exists: ncu
-    cannot run inside the timed program, so the figure is the one of the last capture."""
+    source commit it records for the capture).  ``average``: over the launches with and without
+    x updates, where the file has both.  (None, None) when no capture exists: ncu cannot run
+    inside the timed program, so the figure is the one of the last capture."""
     f = ROOT / 'profiles' / f'{kernel}_{PROFILE_TAGS[workload]}.md'
     if f.exists():
         text = f.read_text()
-        m = re.search(r'traffic_bytes_per_launch:\s*([0-9.eE+]+)', text)
+        m = (average and re.search(r'average_bytes_per_launch:\s*([0-9.eE+]+)', text)) or \
+            re.search(r'traffic_bytes_per_launch:\s*([0-9.eE+]+)', text)
         if m:
             c = re.search(r'captured_source_commit:\s*([0-9a-f]+)', text)
             return float(m.group(1)), f'profiles/{f.name}' + (f' (capture of commit {c.group(1)})' if c else '')
@@ -214,7 +217,9 @@ def run_ours(args) -> dict | None:
     op = GridOperator(p.omega, p.dxes, p.epsilon, p.mu, p.pec, p.pmc, device=dev, fp32=True)
     J = torch.as_tensor(p.J, device=dev)
     stream = torch.cuda.current_stream()
-    tuned = op.autotune(methods=tuple(args.methods.split(','))) if args.autotune else {}
+    # (the iterations of a resident solve have no x chunk to tune)
+    tunable = tuple(m for m in args.methods.split(',') if not op.resident(m))
+    tuned = op.autotune(methods=tunable) if args.autotune and tunable else {}
 
     fields = {}  # the last timed field of each method
 
@@ -243,8 +248,8 @@ def run_ours(args) -> dict | None:
         return max_over_ranks(total_ms, world), lats, infos
 
     # Per-kernel CUDA-event timing inside the timed solves costs two event records per launch
-    # and disables the iteration graphs (about 10 % at 160x160x128, far more on small grids),
-    # so the timed solves run as they do in production (graph launches) and the kernel
+    # and disables the iteration graphs (about 10 % at 160x160x128, far more on small grids)
+    # and the resident form, so the timed solves run as they do in production and the pass
     # durations of the roofline come from one profiled solve per method right after them.
     live = args.timed_profile == 'on'
     out = {}
@@ -314,10 +319,27 @@ def run_ours(args) -> dict | None:
         extra_bytes = (3 * real if p.mu is not None else 0) + (1 if (p.pec is not None or p.pmc is not None) else 0)
     alg = (kernel_bytes(dom, p) + extra_bytes) * ncell
     achieved = alg / (avg_ms / 1e3) / 1e9
-    traffic, traffic_source = profile_traffic(KERNEL_NAMES[dom], args.workload)
-    if traffic_source and kernel_bytes(dom, p) != KERNEL_BYTES_PER_CELL[dom]:
-        traffic_source += ', a launch with x updates (every second one; algorithmic bytes are the average)'
+    # (where only every second launch updates x, bytes and durations are averages)
+    traffic, traffic_source = profile_traffic(KERNEL_NAMES[dom], args.workload,
+                                              average=kernel_bytes(dom, p) != KERNEL_BYTES_PER_CELL[dom])
     share = b['kernel_ms'][dom] / b['prof_ms']
+    resident = op.resident(best) and not live
+    roofline = {'bound': 'hbm', 'kernel': KERNEL_NAMES[dom], 'achieved': round(achieved, 1),
+                'peak': peak, 'unit': 'GB/s', 'frac': round(achieved / peak, 4),
+                'peak_kind': peak_kind, 'traffic': traffic, 'traffic_source': traffic_source,
+                'algorithmic_bytes_per_launch': alg, 'avg_launch_ms': round(avg_ms, 5),
+                'share_of_step': round(share, 3),
+                'timing': ('CUDA events around every launch of the timed solves' if live else
+                           'CUDA events around every launch of one profiled solve after the timed ones, which '
+                           + ('run resident: another form of the same iteration' if resident else
+                              'launch the same passes as graphs'))}
+    if resident:
+        # the kernel that the timed solves run; the passes of the profiled solve beside it
+        roofline = {'bound': 'latency of two grid-wide exchanges per iteration, and shared memory',
+                    'kernel': RESIDENT_NAMES[best], 'achieved': round(1e3 * b['ms_per_step'] / b['iterations'], 3),
+                    'unit': 'us per iteration', 'peak': None, 'frac': None,
+                    'timing': 'CUDA events around the timed solves, set-up and residual check included',
+                    'launch_per_pass_form': roofline}
     steps_total = args.steps
     res = {
         'metric': METRIC, 'value': round(b['solves_per_s'], 4), 'unit': 'solves/s', 'n_gpus': world,
@@ -334,14 +356,7 @@ def run_ours(args) -> dict | None:
                  if 'cocg' in out else None),
         'mixed_over_fp64': (round(out['mixed']['solves_per_s'] / out['cocg']['solves_per_s'], 3)
                             if 'mixed' in out and 'cocg' in out else None),
-        'roofline': {'bound': 'hbm', 'kernel': KERNEL_NAMES[dom], 'achieved': round(achieved, 1),
-                     'peak': peak, 'unit': 'GB/s', 'frac': round(achieved / peak, 4),
-                     'peak_kind': peak_kind, 'traffic': traffic, 'traffic_source': traffic_source,
-                     'algorithmic_bytes_per_launch': alg, 'avg_launch_ms': round(avg_ms, 5),
-                     'share_of_step': round(share, 3),
-                     'timing': ('CUDA events around every launch of the timed solves' if live else
-                                'CUDA events around every launch of one profiled solve after the '
-                                'graph-launched timed solves')},
+        'roofline': roofline,
         'field_rel_err': field_errors(fields, args.workload),
         'gpu_launches': int(b['launches']),
         'tiling': {k: {'xchunk': v[0], 'us_per_iteration': round(v[1], 1)} for k, v in tuned.items()},
