@@ -384,6 +384,7 @@ static int launch_point(fdfd_plan* P, const Geo<R>& g, const Op& op, RedBuf rb, 
 
 // ------------------------------------------------------------------ resident solves
 static constexpr int RES_CHUNK = 256;  // iterations per launch: a millisecond or two between polls
+static constexpr int RES_CHUNK_MAX = 1 << 16;  // counters are 32 bits: CTAs x iterations of a launch
 static constexpr int RES_REFUSED = 1;  // the device does not take the cooperative launch; nothing ran
 
 // The brick split with the least work on the largest brick among those of at most one CTA of
@@ -960,6 +961,9 @@ struct SolveCtx {
   int fallbacks;   // mixed -> complex128 COCG switches
 };
 
+// iterations of one resident launch
+static int resident_chunk(const fdfd_solve_opts* o) { return o->chunk > 0 ? std::min(o->chunk, RES_CHUNK_MAX) : RES_CHUNK; }
+
 static double monitored(const KState& h, int crit) { return crit == 0 ? h.rr : (crit == 1 ? h.rr_pc : h.rr_w2); }
 
 // Refinement loop: r = b - A0 E in complex128 (exact criterion), then an inner
@@ -1039,7 +1043,7 @@ static int refine_loop(SolveCtx& c, const Geo<RI>& gi, int prec, BsBufs B, doubl
       if (resident) {
         Word* surface = (Word*)B.R1;
         if (local_outer == 1) CK(cudaMemsetAsync(surface, 0, 5 * vb, s));
-        const int nit = c.o->chunk > 0 ? c.o->chunk : RES_CHUNK;
+        const int nit = resident_chunk(c.o);
         rc = drive(P, sti, nit, hi.maxiter, s, [&]() -> int {
           if (!c.take_launch()) return RES_REFUSED;
           const unsigned long long tag = c.tag;
@@ -1148,7 +1152,7 @@ static int cocg_loop(SolveCtx& c, cx<double>* r, cx<double>* q, cx<double>* P0, 
     CK(cudaStreamSynchronize(s));
     const int left = maxiter - c.iters;
     if (resident && P->h_state->status == ST_RUNNING && left > 0) {
-      const int nit = o->chunk > 0 ? o->chunk : RES_CHUNK;
+      const int nit = resident_chunk(o);
       rc = drive(P, st, nit, left, s, [&]() -> int {
         if (!c.take_launch()) return RES_REFUSED;
         const unsigned long long tag = c.tag;

@@ -87,3 +87,20 @@ def test_the_cap_holds_when_the_form_changes(problem, limit):
     E, info = op.solve(J, rtol=1e-13, criterion='true', chunk=1, maxiter=7, wait_limit=limit)
     assert (info.status, info.iterations) == ('maxiter', 7)
     assert abs(op.residual(E, J)['rel'] / info.residual - 1) <= 1e-9
+
+
+def test_chunks_are_cut_to_what_the_counters_hold(cuda):
+    """A launch counts CTAs times iterations in 32 bits: a chunk of 2^31 - 1 is cut, with the same
+    bits as the default.  (A count that runs over takes 29 million iterations.)"""
+    from meanas_b200.operators import GridOperator
+    shape = (3, 5, 4)
+    n = 3 * int(numpy.prod(shape))
+    rng = numpy.random.default_rng(3)
+    dxes = [[numpy.ones(m, dtype=complex) for m in shape] for _ in range(2)]
+    op = GridOperator(0.5, dxes, numpy.ones(n), device=cuda)
+    J = rng.standard_normal(n) + 1j * rng.standard_normal(n)
+    kw = dict(rtol=1e-9, criterion='true')
+    E, info = op.solve(J, **kw)
+    big, ibig = op.solve(J, chunk=2 ** 31 - 1, **kw)
+    assert info.converged and ibig.iterations == info.iterations
+    assert numpy.array_equal(big.cpu().numpy(), E.cpu().numpy())
