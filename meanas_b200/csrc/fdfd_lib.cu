@@ -383,7 +383,12 @@ static int launch_point(fdfd_plan* P, const Geo<R>& g, const Op& op, RedBuf rb, 
 }
 
 // ------------------------------------------------------------------ resident solves
-static constexpr int RES_CHUNK = 256;  // iterations per launch: a millisecond or two between polls
+// Iterations per launch.  A launch of whole-SM CTAs and the kernels of a solve on another stream
+// take turns, so it ends before a millisecond; half-SM CTAs run beside such kernels.  Per
+// iteration of 48^3 alone, and of a 160x160x128 solve on another stream meanwhile: 256 iterations
+// 12.7 and 1990 us, 64 12.9 and 1450, 32 13.4 and 1000, 16 14.4 and 700 (one more launch costs 27
+// us).  The same of 128x128 with 256: 6.6 and 440 us.
+static constexpr int RES_CHUNK = 64, RES_CHUNK_HALF = 256;
 static constexpr int RES_CHUNK_MAX = 1 << 16;  // counters are 32 bits: CTAs x iterations of a launch
 static constexpr int RES_REFUSED = 1;  // the device does not take the cooperative launch; nothing ran
 
@@ -420,9 +425,8 @@ static ResidentPlan split_bricks(const fdfd_plan* P, int nshell, int nred, int n
 }
 
 // CTAs of half an SM where bricks of one cell per thread (two on flat grids) cover the grid,
-// otherwise of a whole SM.  A launch of the latter has the GPU to itself for its 256
-// iterations, so solves on other streams take turns with it, while two of the former share the
-// SMs.  Alone / eight at once, us per iteration of the two-launch form before, whole SM, half:
+// otherwise of a whole SM.  A launch of the latter has the GPU to itself, so solves on other
+// streams take turns with it, while two of the former share the SMs.  Alone / eight at once, us per iteration of the two-launch form before, whole SM, half:
 // BiCGSTAB 128x128 30 / 4.7, 6.6 / 6.3, 6.4 / 3.4; 256x256 32 / 6.6, 7.6 / 7.3, 8.1 / 5.0; COCG 24^3
 // 26 / 3.9, 6.3 / 6.0, 6.1 / 3.4; 32^3 27 / 4.7, 7.7 / 7.4, 7.5 / 5.0.  Larger 3D grids gain on whole SMs
 // either way: 36^3 29 / 9.2, 8.2 / 7.9, 11.3 / 6.9 (two cells per thread); 48^3 31 / 16, 12.4 / 12.2, does
@@ -962,7 +966,10 @@ struct SolveCtx {
 };
 
 // iterations of one resident launch
-static int resident_chunk(const fdfd_solve_opts* o) { return o->chunk > 0 ? std::min(o->chunk, RES_CHUNK_MAX) : RES_CHUNK; }
+static int resident_chunk(const ResidentPlan& rp, const fdfd_solve_opts* o) {
+  if (o->chunk > 0) return std::min(o->chunk, RES_CHUNK_MAX);
+  return rp.nt == RES_NT_HALF ? RES_CHUNK_HALF : RES_CHUNK;
+}
 
 static double monitored(const KState& h, int crit) { return crit == 0 ? h.rr : (crit == 1 ? h.rr_pc : h.rr_w2); }
 
@@ -1043,7 +1050,7 @@ static int refine_loop(SolveCtx& c, const Geo<RI>& gi, int prec, BsBufs B, doubl
       if (resident) {
         Word* surface = (Word*)B.R1;
         if (local_outer == 1) CK(cudaMemsetAsync(surface, 0, 5 * vb, s));
-        const int nit = resident_chunk(c.o);
+        const int nit = resident_chunk(P->res_bs, c.o);
         rc = drive(P, sti, nit, hi.maxiter, s, [&]() -> int {
           if (!c.take_launch()) return RES_REFUSED;
           const unsigned long long tag = c.tag;
@@ -1152,7 +1159,7 @@ static int cocg_loop(SolveCtx& c, cx<double>* r, cx<double>* q, cx<double>* P0, 
     CK(cudaStreamSynchronize(s));
     const int left = maxiter - c.iters;
     if (resident && P->h_state->status == ST_RUNNING && left > 0) {
-      const int nit = resident_chunk(o);
+      const int nit = resident_chunk(P->res_cocg, o);
       rc = drive(P, st, nit, left, s, [&]() -> int {
         if (!c.take_launch()) return RES_REFUSED;
         const unsigned long long tag = c.tag;

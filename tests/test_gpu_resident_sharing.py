@@ -123,3 +123,19 @@ def test_solves_at_once_give_the_same_bits(cuda):
             t.join()
         for k in range(len(jobs)):
             assert numpy.array_equal(alone[k], together[k]), k
+
+
+@pytest.mark.parametrize('method', ['cocg', 'mixed'])
+@pytest.mark.parametrize('shape,most', [((40, 40, 40), 64), ((30, 30, 30), 256)], ids=str)
+def test_whole_sm_launches_are_short(cuda, shape, method, most):
+    """Launches that have the GPU to themselves end after 64 iterations, so that kernels of other
+    streams get their turn; the result does not depend on it."""
+    from meanas_b200.operators import GridOperator
+    p, J, _ = _problem(shape, False)
+    op = GridOperator(**p, device=cuda)
+    kw = dict(method=method, rtol=1e-13, criterion='true', maxiter=512, max_outer=1, inner_rtol=1e-12)
+    E, info = op.solve(J, **kw)
+    # two launches are under way when a solve ends, and about ten kernels come before and after
+    assert 512 // most <= info.kernel_launches <= 512 // most + 15
+    other, _ = op.solve(J, chunk=100, **kw)
+    assert numpy.array_equal(other.cpu().numpy(), E.cpu().numpy())
