@@ -264,7 +264,8 @@ __device__ __forceinline__ void fdtd_cells(const FdtdGeo& g, const double2* tab,
 // H / E half step before and now, 160x160x128: float32 51 / 84 -> 35 / 50 us (PLAIN), 78 / 100 ->
 // 59 / 65 (CPML on every face); float64 93 / 103 -> 47 / 53, 115 / 124 -> 60 / 64; flat
 // 1000x800 float32 454 / 525 -> 19 / 21.  Four CTAs of 64 registers per SM: three or five are 2
-// to 15 % slower.
+// to 15 % slower.  The instances with layers (FACES 1) spill 130 to 240 bytes per thread at
+// that cap, the others next to nothing.
 template <typename R, typename P, bool ESTEP, int FACES, bool TABLE>
 __global__ void __launch_bounds__(FDTD_NT, 4) k_fdtd(const FdtdGeo g, R* __restrict__ e, R* __restrict__ h) {
   __shared__ double2 tab[TABLE ? FDTD_TABLE : 1];

@@ -1135,8 +1135,9 @@ static int cocg_loop(SolveCtx& c, cx<double>* r, cx<double>* q, cx<double>* P0, 
     }
     return 0;
   };
-  // Every grid that fits runs resident: it is 2 to 4 times faster than the two launches up to
-  // the largest that do (52^3 and 380^2 cells, see k_cocg_resident).  The two-launch form
+  // Every grid that fits runs resident: alone it is 1.9 to 3.7 times faster than the two launches
+  // up to the largest that do (52^3 and 380^2 cells, see k_cocg_resident), and with others in
+  // flight faster too (see plan_resident).  The two-launch form
   // stays for larger grids, for profiling (which times its passes) and where the caller's
   // workspace has no room for the surface words (the fallback of the mixed solver), and takes
   // over where a cooperative launch is refused or a wait in one ran out.

@@ -554,11 +554,11 @@ __host__ __device__ inline ResidentLayout resident_layout(int nshell, int nred, 
 // thread in registers.  `surface`: two buffers (even and odd tags) of 6 N words, since the
 // shell is read while the second exchange is under way.
 //
-// Measured per iteration, two launches / resident: 16^3 25.0 / 5.9 us, 40^3 28.5 / 9.9, 52^3
-// (the largest cube that fits) 37.4 / 16.9; flat 128^2 23.4 / 6.1, 380^2 34.2 / 11.0.  It is
+// Measured per iteration, two launches / resident: 16^3 20.8 / 5.6 us, 32^3 21.9 / 7.3, 40^3
+// 23.0 / 10.2, 52^3 (the largest cube that fits) 32.5 / 17.4; flat 128^2 20.0 / 5.5, 380^2 31.5 / 11.3.  It is
 // bound by the exchanges (about 3 us of each iteration) and, on full bricks, by shared-memory
-// bandwidth in the two curl passes.  Of that, dividing by reciprocals (cdiv), block sums through
-// shared memory and material code by template gave 0.4 to 0.8 us.
+// bandwidth in the two curl passes.  Dividing by reciprocals (cdiv), block sums through shared
+// memory and material code by template gave 0.4 to 0.7 us of it.
 constexpr int COCG_SUMS = 5;
 template <int NT, int K, bool FLAT, bool MAT>
 __global__ void __launch_bounds__(NT, RES_NT / NT)
@@ -786,8 +786,8 @@ __global__ void __launch_bounds__(NT, RES_NT / NT)
 // shells are read before the sums that their writers wait for, so each product has one
 // buffer of 3 N words.
 //
-// Measured per iteration, two launches / resident: 16^3 29.6 / 6.8 us, 40^3 33.6 / 9.5, 52^3
-// (the largest cube that fits) 44.2 / 14.0; flat 128^2 29.7 / 6.7, 380^2 39.6 / 9.9.
+// Measured per iteration, two launches / resident: 16^3 26.8 / 6.3 us, 32^3 28.6 / 8.4, 40^3
+// 30.1 / 9.8, 52^3 (the largest cube that fits) 39.5 / 14.4; flat 128^2 25.6 / 6.2, 380^2 35.6 / 10.2.
 // Bound as COCG is: two exchanges, then shared-memory bandwidth on full bricks.
 constexpr int BS_SUMS = 6;
 template <int NT, int K, bool FLAT, bool MAT>
